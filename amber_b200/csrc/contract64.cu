@@ -35,7 +35,7 @@ struct F64Desc {
     const int *groups;           // anchor groups, concatenated over anchor blocks
     const int *group_off;        // [nab + 1]
     long k, kp;
-    int nc, nc10, nclen, ks, AB;
+    int nc, nc10, nclen, ks, rs, AB;
 };
 
 constexpr int F_S1 = LS_SPAN + 1;  // D1 rows of an anchor block (≤ 256)
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(F_NT, 1) ls_fp64_kernel(const F64Desc *__restr
     const int gq = lane >> 2, tq = lane & 3;   // fragment row / column group, k index
     const int ks = j.ks, nclen = j.nclen, nc = j.nc;
     const int c0 = u.ab * j.AB, c1 = min(nc, c0 + j.AB), nab1 = c1 - c0;
-    const int mrows = ks > 1 ? ks * nclen : min(LS_ROWS, nclen - LS_ROWS * u.t3);
+    const int mrows = ks > 1 ? ks * j.rs : min(LS_ROWS, nclen - LS_ROWS * u.t3);
     const int ncols = ks > 1 ? nclen + ks - 1 : min(LS_ROWS, nclen - LS_ROWS * u.t2);
     const int row0_3 = c0 - j.nc10 + (ks > 1 ? 0 : LS_ROWS * u.t3);  // channel of staged D3 row 0
     const int row0_2 = c0 - j.nc10 + (ks > 1 ? 0 : LS_ROWS * u.t2);  // channel of staged D2 row 0
@@ -80,8 +80,8 @@ __global__ void __launch_bounds__(F_NT, 1) ls_fp64_kernel(const F64Desc *__restr
     const int g0 = j.group_off[u.ab], g1 = j.group_off[u.ab + 1];
     // the A row this thread forms (pixels tid/128 + 4i), its anchor slot and lag
     const int ar = tid & (LS_ROWS - 1), ax = tid >> 7;
-    const int aslot = ks > 1 ? ar / nclen : 0, ad3 = ks > 1 ? ar % nclen : ar;
-    const bool arow = ar < mrows;
+    const int aslot = ks > 1 ? ar / j.rs : 0, ad3 = ks > 1 ? ar % j.rs : ar;
+    const bool arow = ar < mrows && ad3 < nclen;
 
     double acc[2][4][4];
 #pragma unroll
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(F_NT, 1) ls_fp64_kernel(const F64Desc *__restr
         for (int hr = 0; hr < 2; ++hr) {
             const int r = 32 * wm + 16 * mt + 8 * hr + gq;
             if (r >= mrows) continue;
-            const int a = ks > 1 ? r / nclen : 0;
+            const int a = ks > 1 ? r / j.rs : 0;
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
@@ -345,13 +345,13 @@ int contract_fp64_jobs(amber_cuda_ctx *c, const std::vector<F64Job> &jobs)
             x.groups = (const int *)(d + off_g) + gpos;
             x.group_off = (const int *)(d + off_o) + opos;
             x.k = jb.k; x.kp = jb.kp;
-            x.nc = (int)c->nc; x.nc10 = c->nc10; x.nclen = nclen; x.ks = p.s.k; x.AB = p.s.AB;
+            x.nc = (int)c->nc; x.nc10 = c->nc10; x.nclen = nclen; x.ks = p.s.k; x.rs = p.s.rs; x.AB = p.s.AB;
             std::copy(p.groups.begin(), p.groups.end(), hg + gpos);
             for (size_t q = 0; q < p.group_off.size(); ++q) ho[opos + q] = p.group_off[q];
             gpos += p.groups.size();
             opos += p.group_off.size();
             red.push_back(LsReduceJob{(const double *)c->partial.p + p.unit_base * LS_ROWS * LS_ROWS, jb.lag_out, nclen,
-                                      p.s.k, p.s.T, p.s.nab, p.s.V});
+                                      p.s.k, p.s.rs, p.s.T, p.s.nab, p.s.V});
         }
         std::copy(units.begin(), units.end(), (LsUnit *)(h + off_u));
         if ((rc = cuda_check(c, cudaMemcpyAsync(d, h, stage_b, cudaMemcpyHostToDevice, c->stream), "job list upload")))

@@ -40,13 +40,32 @@
 // fp32 D1 rows of its anchor block and the D2 digits of its window span, and
 // then runs every anchor group of the block against them.
 //
-// Warp roles (576 threads): warps 0-15 form the A digits (warp w: TMEM lanes
-// 32·(w mod 4) .. +31, pixels 8·(w div 4) .. +7 of the slice) and run each
-// block's epilogue; warp 16 streams the slices by TMA; warp 17 owns TMEM and
-// issues the MMAs from one lane.  Four A buffers let the formers run ahead of
-// the tensor pipe.  Every mbarrier wait is bounded; on expiry the CTA raises an
+// Warp roles (640 threads): warps 0-15 form the A digits (four sets of four
+// warps, each set a whole anchor group, warp w the TMEM lanes 32·(w mod 4) .. +31)
+// and run each block's epilogue; warp 16 streams the slices by TMA; warps 17 and
+// 18 issue the MMAs, one elected thread each, into accumulators of their own;
+// warp 19 scales the staged D1 rows.  Five or more A buffers let the formers run
+// ahead of the tensor pipe.  Every wait is bounded; on expiry the CTA raises an
 // error flag the host turns into AMBER_ERR_TIMEOUT, drains its own copies and
 // MMAs and frees TMEM.  No cluster launch and no multicast.
+//
+// What bounds it, and what it measured (one CTA per SM, cycles per anchor group
+// and 32-pixel slice on the Ng1 = 740 maps, 128 channels, nclen = 127; triangles
+// of that size took 6.14 ms each before and 3.65 ms now):
+//   * 932 before.  The six MMAs of a group need 384 cycles at N = 128 (N/2 each,
+//     42 at least), 312 over the channel range alone.  The issuing warp was the
+//     bound: an mbarrier wait per group, operands the compiler did not know to be
+//     uniform (a register-to-uniform move each), and issue slots shared with the
+//     formers.  Counts in place of barriers, one elected thread per issuing warp,
+//     operands from a table and two issuing warps took it to 362 with the formers'
+//     arithmetic switched off.
+//   * The formers are the bound now: ~290 instructions per warp and group at 64 %
+//     of the issue slots.  A packed FP32x2 op with three different 64-bit operands
+//     costs 3.3 cycles against 1.0 for a scalar one and PRMT costs 2, so packed
+//     ops save issue slots rather than pipe time: all-scalar digits were 8 % slower.
+//   * Blocks of 8 rows outside the channel range are skipped (a quarter of them at
+//     nc10 = nc/2 − 1, half at nc − 1).  12 or 20 former warps in place of 16
+//     (128 or 80 registers each) were 8 % and 6 % slower.
 #include <string.h>
 
 #include <algorithm>
@@ -66,23 +85,23 @@ using namespace tc;
 constexpr int SLICE = 32;                    // pixels per K step (one kind::i8 MMA)
 constexpr int NSLICE = LS_BLOCK / SLICE;     // slices per block
 constexpr int NFORM = 16;                    // former / epilogue warps
-constexpr int WARP_TMA = 16, WARP_MMA = 17;
-constexpr int NTHREADS = 18 * 32;
+constexpr int WARP_TMA = NFORM, WARP_MMA = NFORM + 1, WARP_MMA2 = NFORM + 2, WARP_SCALE = NFORM + 3;
+constexpr int NMMA = 2;                      // MMA issuing warps
+constexpr int NTHREADS = (NFORM + 4) * 32;
 constexpr int TMEM_COLS = 512;
-constexpr int ACC_STRIDE = 128;              // TMEM columns per class accumulator
-constexpr int NABUF = 5;                     // A buffers
-constexpr int NSET = 4;                      // former sets: each anchor group is formed by one set of 4 warps
+constexpr int NSET = NFORM / 4;              // former sets: each anchor group is formed by one set of 4 warps
 constexpr int ABUF_COLS = 24;                // 3 digits × 8 columns (32 int8 per row per digit)
-constexpr int A_COL0 = 3 * ACC_STRIDE;       // first A buffer column
-static_assert(A_COL0 + NABUF * ABUF_COLS <= TMEM_COLS, "TMEM");
+constexpr int NABUF_MAX = 8;                 // A buffers: as many as TMEM holds beside the accumulators
+constexpr int NSTAGE_MAX = 8;                // stages: as many as shared memory holds
+static_assert(3 * LS_ROWS + 5 * ABUF_COLS <= TMEM_COLS, "TMEM: five A buffers beside the widest accumulators");
 
-// One stage (one 32-pixel slice) in shared memory, at fixed offsets sized for the largest boxes:
-constexpr int ST_D3 = 0;                     // fp32 D3 rows, 128 B each, 128B swizzle (≤ LS_SPAN rows)
-constexpr int ST_D1 = LS_SPAN * 128;         // fp32 D1 rows of the anchor block, 128 B each
-constexpr int ST_D2 = ST_D1 + LS_SPAN * 128; // D2 digits [3][2][span2][16]
-constexpr int ST_BYTES = ST_D2 + 3 * 2 * LS_SPAN * 16;
-constexpr int NSTAGE = 2;
-static_assert(ST_BYTES % 1024 == 0, "stages keep the 1024-byte alignment of the 128B swizzle");
+// Shared memory: barriers, hand-off counts and the unit's anchor groups, then the stages.
+constexpr int SM_FLAGS = 512;                // [NABUF_MAX] hand-off counts of the A buffers
+constexpr int SM_GROUPS = 768;               // [LS_SPAN + 1] anchor groups (uint4)
+constexpr int SM_STAGES = 5 * 1024;
+constexpr int SMEM_STAGES = 220 * 1024;      // bytes of all stages
+static_assert(SM_GROUPS + 16 * (LS_SPAN + 1) <= SM_STAGES, "group table");
+constexpr size_t SMEM_BYTES = 1024 + (size_t)SM_STAGES + SMEM_STAGES;
 
 struct alignas(64) I8Desc {
     CUtensorMap t3;  // w·D3 fp32 {k, nc}, box {32, span3}, 128B swizzle
@@ -91,35 +110,38 @@ struct alignas(64) I8Desc {
     const int *e1, *e2, *e3;        // block exponents
     const int *groups, *group_off;  // anchor groups of every anchor block
     long k;
-    int nc, nc10, nclen, ks, AB, T;
+    int nc, nc10, nclen, ks, rs, AB, T;
     int span3, span2;
     int sweeps;                     // 1: classes 0-2; 2: also class 3 (mask maps)
     uint32_t tx_bytes;              // bytes one slice's three TMA boxes deliver
+    int nst, st_bytes, st_d1, st_d2;  // stages, bytes of one, offsets of its D1 rows and D2 digits (D3 first)
 };
 
-// Three or four base-254 digits of two products u·v at once (packed FP32x2):
-// every step is one fused op on a pair, the product enters the first rounding
-// unrounded (y0 = fma(u, v, M)), and round-to-nearest through the 1.5·2^23
-// magic number leaves each digit's two's-complement byte in the low mantissa
-// bits.  M − y = −digit exactly, and each residual 254·s − d is exact in FP32
-// (its lowest bit is at most 2^−22 and it is at most 1/2 in magnitude).
+__device__ __forceinline__ float2 sub2(float2 a, float2 b)
+{
+    float2 r;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tsub.rn.f32x2 z, x, y;\n\t"
+        "mov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+
+// Three or four base-254 digits of two products u·v at once (packed FP32x2): the product enters the
+// first rounding unrounded (y0 = fma(u, v, M)), and round-to-nearest through the 1.5·2^23 magic number
+// leaves each digit's two's-complement byte in the low mantissa bits.  M − y = −digit exactly; each
+// residual s = 254·s − d is one fused op.  Only M and 254 are held in registers: a third 64-bit operand
+// costs a packed op a third cycle of register reads, and more constants cost moves.
 template <int ND>
 __device__ __forceinline__ void digits254x2(float2 u, float2 v, float2 (&y)[4])
 {
-    const float2 M = make_float2(12582912.0f, 12582912.0f);
-    const float2 K254 = make_float2(254.f, 254.f);
-    const float2 NEG1 = make_float2(-1.f, -1.f);
-    y[0] = __ffma2_rn(u, v, M);                    // M + d0
-    const float2 nq0 = __ffma2_rn(y[0], NEG1, M);  // −d0
-    const float2 r0 = __ffma2_rn(u, v, nq0);       // u·v − d0
-    y[1] = __ffma2_rn(r0, K254, M);                // M + d1
-    const float2 nq1 = __ffma2_rn(y[1], NEG1, M);  // −d1
-    const float2 s1 = __ffma2_rn(r0, K254, nq1);   // 254·r0 − d1
-    y[2] = __ffma2_rn(s1, K254, M);                // M + d2
-    if constexpr (ND == 4) {
-        const float2 nq2 = __ffma2_rn(y[2], NEG1, M);  // −d2
-        const float2 s2 = __ffma2_rn(s1, K254, nq2);   // 254·s1 − d2
-        y[3] = __ffma2_rn(s2, K254, M);                // M + d3
+    const float2 M = make_float2(12582912.0f, 12582912.0f), K = make_float2(254.f, 254.f);
+    y[0] = __ffma2_rn(u, v, M);                          // M + d0
+    float2 s = __ffma2_rn(u, v, sub2(M, y[0]));          // u·v − d0
+#pragma unroll
+    for (int i = 1; i < ND; ++i) {
+        y[i] = __ffma2_rn(s, K, M);                      // M + di
+        s = __ffma2_rn(s, K, sub2(M, y[i]));             // 254·s − di
     }
 }
 
@@ -129,9 +151,10 @@ __device__ __forceinline__ uint32_t pack_low_bytes(float a, float b, float c, fl
                        __byte_perm(__float_as_uint(c), __float_as_uint(d), 0x0040), 0x5410);
 }
 
-__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t (&v)[4])
+// 16 lanes × 8 columns: lane t/4 and t/4 + 8, column t%4 (v[0], v[1]) and 4 + t%4 (v[2], v[3]) of thread t
+__device__ __forceinline__ void tmem_st16x8(uint32_t taddr, const uint32_t (&v)[4])
 {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x2.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
                  "r"(v[2]), "r"(v[3])
                  : "memory");
 }
@@ -154,30 +177,26 @@ __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, u
         : "memory");
 }
 
-// kind::i8 MMA, A from TMEM, issued by the lane elect.sync picks from the converged MMA warp (every
-// operand is warp-uniform, so the issue costs one instruction), with the accumulate operand as an
-// immediate: the first MMA into an accumulator overwrites it, the rest add.
-__device__ __forceinline__ void umma_i8_set(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc)
+// One kind::i8 MMA (A from TMEM) and one commit, issued by the MMA warps' elected thread.  The operands
+// live in uniform registers there; the descriptor's upper half is the same for every window.  ADD 0
+// overwrites the accumulator's columns.
+template <int ADD>
+__device__ __forceinline__ void umma_i8(uint32_t d, uint32_t a, uint32_t qlo, uint32_t qhi, uint32_t idesc)
 {
-    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
-                 "@e tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, 0;\n\t}" ::"r"(d_tmem), "r"(a_tmem),
-                 "l"(b_desc), "r"(idesc)
+    asm volatile("{\n\t.reg .b64 q;\n\tmov.b64 q, {%2, %3};\n\t"
+                 "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], q, %4, %5;\n\t}" ::"r"(d),
+                 "r"(a), "r"(qlo), "r"(qhi), "r"(idesc), "n"(ADD)
                  : "memory");
 }
-__device__ __forceinline__ void umma_i8_add(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc)
+__device__ __forceinline__ void umma_commit_bar(uint32_t bar)
 {
-    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
-                 "@e tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, 1;\n\t}" ::"r"(d_tmem), "r"(a_tmem),
-                 "l"(b_desc), "r"(idesc)
-                 : "memory");
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-// tcgen05.commit from the elected lane of the converged warp
-__device__ __forceinline__ void umma_commit_elect(uint64_t *bar)
+__device__ __forceinline__ bool elect_one()
 {
-    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
-                 "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
-                     smem_u32(bar))
-                 : "memory");
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e != 0;
 }
 
 // Shared-memory descriptor of a K-major operand without swizzle: 8-row core matrices of
@@ -192,46 +211,191 @@ __device__ __forceinline__ uint64_t smem_desc_plain(uint32_t saddr, uint32_t lbo
     return d;                                    // swizzle mode 0: none
 }
 
+__device__ __forceinline__ float4 lds128(uint32_t a)
+{
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+
+// Hand-off count of an A buffer: its set's four former warps add one each per use.  Relaxed counts
+// between the tcgen05 fences are the hand-off the tensor unit needs; an mbarrier wait or an acquire
+// load here holds the queued MMAs back by ~70 cycles a group.
+__device__ __forceinline__ uint32_t count_load(uint32_t a)
+{
+    uint32_t v;
+    asm volatile("ld.relaxed.cta.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void count_add(uint32_t a)
+{
+    asm volatile("red.relaxed.cta.shared.add.u32 [%0], 1;" ::"r"(a) : "memory");
+}
+__device__ __noinline__ bool count_wait(uint32_t a, uint32_t need, volatile int *abort_flag, int *err, int code)
+{
+    const long long t0 = clock64();
+    while (count_load(a) < need) {
+        if (*abort_flag) return false;
+        if (clock64() - t0 > WAIT_CYCLES) {
+            *abort_flag = 1;
+            atomicExch(err, code);
+            return false;
+        }
+    }
+    return true;
+}
+__device__ __forceinline__ uint4 lds_u128(uint32_t a)
+{
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
+
+// What one MMA issuing thread keeps between its items.
+struct IssueState {
+    uint32_t groups, ngr;          // table of anchor groups (shared address), its length
+    uint32_t acc, nmma, a_first;   // TMEM: this thread's first accumulator, accumulator stride, A buffers
+    uint32_t desc_lo, desc_hi, ddig, stage16;  // D2 descriptor of stage 0, next digit, next stage (16-byte units)
+    uint32_t flags, bars, nabuf;   // hand-off counts and ab_empty barriers (shared addresses)
+    uint32_t ab, need, seen;       // current A buffer, the count that means formed, the count last seen
+    uint32_t s, ph, nst;           // current stage, its parity, stages
+};
+
+// Issues the MMAs of one item (a pixel block, one sweep): every slice's anchor groups in order.
+// SECOND: which of the two issuing threads; class k = Σ_{i+j=k} Q_i·P_j.  SWEEP 0: classes 0 and 1 (first
+// thread) or 2 (second), the A buffer holds P0, P1, P2.  SWEEP 1: class 3 = P3·Q0 + P2·Q1 (first) + P1·Q2
+// (second), the A buffer holds P1, P2, P3.  The loop is kept to few instructions beside the MMAs: they
+// wait for issue slots behind the formers of the same SM partition.
+template <bool SECOND, int SWEEP>
+__device__ __forceinline__ bool issue_item(IssueState &t, int nsl, uint64_t *st_full, uint64_t *st_empty,
+                                           volatile int *abort_flag, int *err)
+{
+    bool first = true;
+    for (int sl = 0; sl < nsl; ++sl) {
+        if (!mbar_wait(&st_full[t.s], t.ph, abort_flag, err, 33)) return false;
+        const uint32_t sd = t.desc_lo + t.s * t.stage16;
+        // the first group of an item sets every column of the accumulators: the table's last entry
+        uint4 e = lds_u128(first ? t.groups + 16 * t.ngr : t.groups);
+        uint32_t next = t.groups;
+        for (uint32_t g = 0; g < t.ngr; ++g) {
+            const uint32_t q0 = sd + e.x, q1 = q0 + t.ddig, q2 = q1 + t.ddig;
+            const uint32_t d = t.acc + e.y, idesc = e.z, a = t.a_first + t.ab * ABUF_COLS;
+            const uint32_t bar = t.bars + t.ab * 8;
+            next += 16;
+            e = lds_u128(next);
+            if (t.seen < t.need && !count_wait(t.flags + t.ab * 4, t.need, abort_flag, err, 34)) return false;
+            fence_after();
+            if (++t.ab == t.nabuf) { t.ab = 0; t.need += 4; }
+            t.seen = count_load(t.flags + t.ab * 4);
+            if (first) {
+                if constexpr (SWEEP == 0 && !SECOND) {
+                    umma_i8<0>(d, a, q0, t.desc_hi, idesc);
+                    umma_i8<0>(d + t.nmma, a + 8, q0, t.desc_hi, idesc);
+                } else {
+                    umma_i8<0>(d, SECOND && SWEEP ? a : a + 16, SECOND && SWEEP ? q2 : q0, t.desc_hi, idesc);
+                }
+                first = false;
+            } else {
+                if constexpr (SWEEP == 0 && !SECOND) {
+                    umma_i8<1>(d, a, q0, t.desc_hi, idesc);
+                    umma_i8<1>(d + t.nmma, a + 8, q0, t.desc_hi, idesc);
+                } else {
+                    umma_i8<1>(d, SECOND && SWEEP ? a : a + 16, SECOND && SWEEP ? q2 : q0, t.desc_hi, idesc);
+                }
+            }
+            if constexpr (SWEEP == 0 && !SECOND) umma_i8<1>(d + t.nmma, a, q1, t.desc_hi, idesc);
+            if constexpr (SWEEP == 0 && SECOND) {
+                umma_i8<1>(d, a + 8, q1, t.desc_hi, idesc);
+                umma_i8<1>(d, a, q2, t.desc_hi, idesc);
+            }
+            if constexpr (SWEEP == 1 && !SECOND) umma_i8<1>(d, a + 8, q1, t.desc_hi, idesc);
+            umma_commit_bar(bar);
+        }
+        umma_commit_bar(smem_u32(&st_empty[t.s]));
+        if (++t.s == t.nst) { t.s = 0; t.ph ^= 1; }
+    }
+    return true;
+}
+
 __global__ void __launch_bounds__(NTHREADS, 1)
     ls_i8_kernel(const I8Desc *__restrict__ jobs, const LsUnit *__restrict__ units, double *__restrict__ partial,
                  int *err)
 {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + NSTAGE * ST_BYTES);
-    uint64_t *st_full = bars, *st_empty = st_full + NSTAGE;
-    uint64_t *ab_full = st_empty + NSTAGE, *ab_empty = ab_full + NABUF;
-    uint64_t *acc_full = ab_empty + NABUF, *acc_empty = acc_full + 1, *drain = acc_empty + 1;
-    volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(drain + 1);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
+    uint64_t *st_full = bars, *st_ready = st_full + NSTAGE_MAX, *st_empty = st_ready + NSTAGE_MAX;
+    uint64_t *ab_empty = st_empty + NSTAGE_MAX;
+    uint64_t *acc_full = ab_empty + NABUF_MAX, *acc_empty = acc_full + 1, *drain = acc_empty + 1;
+    volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(drain + NMMA);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    int *sgroups = reinterpret_cast<int *>(smem + NSTAGE * ST_BYTES + 256);  // this anchor block's groups
-    unsigned char *zero_row = smem + NSTAGE * ST_BYTES + 256 + sizeof(int) * LS_SPAN;  // 128 zero bytes
+    int *ngroups_s = reinterpret_cast<int *>(smem + SM_FLAGS - 4);
+    uint32_t *ab_flags = reinterpret_cast<uint32_t *>(smem + SM_FLAGS);
+    uint4 *sgroups = reinterpret_cast<uint4 *>(smem + SM_GROUPS);
+    unsigned char *stages = smem + SM_STAGES;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const LsUnit u = units[blockIdx.x];
     const I8Desc *jd = jobs + u.job;
-    const int g0 = jd->group_off[u.ab], g1 = jd->group_off[u.ab + 1];
-    const int ks = jd->ks, nclen = jd->nclen, nc = jd->nc;
+    const int ks = jd->ks, nclen = jd->nclen, nc = jd->nc, nc10 = jd->nc10, rs = jd->rs;
     const int c0 = u.ab * jd->AB, c1 = min(nc, c0 + jd->AB);
-    const int mrows = ks > 1 ? ks * nclen : min(LS_ROWS, nclen - LS_ROWS * u.t3);
-    const int ncols = ks > 1 ? nclen : min(LS_ROWS, nclen - LS_ROWS * u.t2);  // lag columns
-    const int nmma = ks > 1 ? ((nclen + ks - 1 + 15) / 16) * 16 : ((ncols + 15) / 16) * 16;  // MMA N
+    const int toff3 = ks > 1 ? 0 : LS_ROWS * u.t3, toff2 = ks > 1 ? 0 : LS_ROWS * u.t2;
+    const int mrows = ks > 1 ? ks * rs : min(LS_ROWS, nclen - toff3);
+    const int ncols = ks > 1 ? nclen : min(LS_ROWS, nclen - toff2);  // lag columns
+    const int nwin = ks > 1 ? nclen + ks - 1 : ncols;                // window rows of D2
+    const int nmma = ((nwin + 15) / 16) * 16;                        // MMA N
+    const int nabuf = min(NABUF_MAX, (TMEM_COLS - 3 * nmma) / ABUF_COLS);
+    const int nst = jd->nst, st_bytes = jd->st_bytes;
     double *out = partial + u.tile * (long)(LS_ROWS * LS_ROWS);
 
-    if (g1 == g0) {
-        // an anchor block without anchors contributes nothing: its partial tile is zero
-        for (int e = tid; e < LS_ROWS * LS_ROWS; e += NTHREADS) out[e] = 0.0;
-        return;
+    // The unit's anchor groups {D2 descriptor offset, accumulator column, MMA instruction descriptor,
+    // 16 × staged row of the first channel and mask of live 8-row blocks}.  Columns whose D2 channel lies outside [0, nc) add nothing, so a group's
+    // MMAs run over its own channel range only (whole 16-column steps), and a group with no channel in
+    // range at all (a corner tile of a wide window) is dropped.  The entry after the last is the first
+    // group over all columns, which sets the accumulators.
+    if (warp == 0) {
+        // S32 accumulate, signed int8 A and B, both K-major, M = 128, N / 8 in bits 17-22
+        const uint32_t idesc0 = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(LS_ROWS >> 4) << 24);
+        const int g0 = jd->group_off[u.ab], g1 = jd->group_off[u.ab + 1];
+        int n = 0;
+        for (int gb = g0; gb < g1; gb += 32) {
+            const int pb = gb + lane < g1 ? jd->groups[gb + lane] : 0;
+            const int w2 = pb - nc10 + toff2, w3 = pb - nc10 + toff3;  // channels of the first column and row
+            const int lo = max(0, -w2), hi = min(nwin, nc - w2);
+            const bool keep = gb + lane < g1 && lo < hi && (ks > 1 || (w3 < nc && w3 + mrows > 0));
+            const unsigned m = __ballot_sync(0xffffffffu, keep);
+            const int at = n + __popc(m & ((1u << lane) - 1u));
+            const uint32_t row = (uint32_t)(pb - c0), col = (uint32_t)(lo / 16) * 16;
+            // 8-row blocks of the tile with a row whose D3 channel (and anchor) is in range, bits 16-31
+            uint32_t blocks = 0;
+            for (int a = 0; a < ks && pb + a < c1; ++a) {
+                const int ra = max(0, -(w3 + a)), rb = min(ks > 1 ? nclen : mrows, nc - (w3 + a));  // its lags in range
+                if (ra < rb)
+                    blocks |= (0xffffu << ((a * rs + ra) / 8)) & (0xffffu >> (15 - (a * rs + rb - 1) / 8));
+            }
+            if (keep)
+                sgroups[at] = make_uint4(row + col, col, idesc0 | (((hi + 15) / 16) * 2u - col / 8) << 17,
+                                         16 * row | blocks << 16);
+            n += __popc(m);
+        }
+        __syncwarp();
+        if (lane == 0) {
+            *ngroups_s = n;
+            const uint32_t row = n > 0 ? (sgroups[0].w & 0xffffu) / 16 : 0u;
+            sgroups[n] = make_uint4(row, 0u, idesc0 | (uint32_t)(nmma / 8) << 17, 0u);
+        }
     }
-
-    for (int i = tid; i < g1 - g0; i += NTHREADS) sgroups[i] = jd->groups[g0 + i];
-    if (tid < 32) reinterpret_cast<uint32_t *>(zero_row)[tid] = 0u;
+    if (tid < NABUF_MAX) ab_flags[tid] = 0u;
     if (tid == 0) {
-        for (int s = 0; s < NSTAGE; ++s) { mbar_init(&st_full[s], 1); mbar_init(&st_empty[s], NFORM + 1); }
-        for (int s = 0; s < NABUF; ++s) { mbar_init(&ab_full[s], NFORM / NSET); mbar_init(&ab_empty[s], 1); }
-        mbar_init(acc_full, 1);
+        for (int s = 0; s < NSTAGE_MAX; ++s) {
+            mbar_init(&st_full[s], 1);
+            mbar_init(&st_ready[s], 1);
+            mbar_init(&st_empty[s], NFORM + NMMA);
+        }
+        for (int s = 0; s < NABUF_MAX; ++s) mbar_init(&ab_empty[s], NMMA);
+        mbar_init(acc_full, NMMA);
         mbar_init(acc_empty, NFORM);
-        mbar_init(drain, 1);
+        for (int s = 0; s < NMMA; ++s) mbar_init(&drain[s], 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -245,6 +409,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tmem_slot;
+    const uint32_t a_col0 = tmem + 3 * nmma;
+    const int ngr = *ngroups_s;
     bool ok = true;
     const int sweeps = jd->sweeps;
     const long k = jd->k;
@@ -253,209 +419,239 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         return (int)(n < NSLICE ? n : NSLICE);
     };
 
-    if (warp == WARP_TMA) {
+    if (ngr == 0) {
+        // no anchor of the block has a channel in range: the partial tile is zero
+        for (int e = tid; e < LS_ROWS * LS_ROWS; e += NTHREADS) out[e] = 0.0;
+    } else if (warp == WARP_TMA) {
         if (lane == 0) {
-            const int row0_3 = c0 - jd->nc10 + (ks > 1 ? 0 : LS_ROWS * u.t3);
-            const int row0_2 = c0 - jd->nc10 + (ks > 1 ? 0 : LS_ROWS * u.t2);
-            int ns = 0;
+            const int row0_3 = c0 - nc10 + toff3, row0_2 = c0 - nc10 + toff2;
+            const int st_d1 = jd->st_d1, st_d2 = jd->st_d2;
+            int ns = 0, s = 0, ph = 1;
             for (long b = u.b0; b < u.b1 && ok; ++b)
                 for (int sw = 0; sw < sweeps && ok; ++sw)
                     for (int sl = 0; sl < nslices(b); ++sl, ++ns) {
-                        const int s = ns % NSTAGE;
-                        if (!mbar_wait(&st_empty[s], ((ns / NSTAGE) & 1) ^ 1, abort_flag, err, 31)) { ok = false; break; }
-                        unsigned char *st = smem + s * ST_BYTES;
+                        if (!mbar_wait(&st_empty[s], ph, abort_flag, err, 31)) { ok = false; break; }
+                        unsigned char *st = stages + s * st_bytes;
                         mbar_expect_tx(&st_full[s], jd->tx_bytes);
                         const int x = (int)(b * LS_BLOCK + sl * SLICE);
-                        tma_load_2d(st + ST_D3, &jd->t3, &st_full[s], x, row0_3);
-                        tma_load_2d(st + ST_D1, &jd->t1, &st_full[s], x, c0);
-                        tma_load_4d(st + ST_D2, &jd->t2, &st_full[s], 0, row0_2, x / 16, 0);
+                        tma_load_2d(st, &jd->t3, &st_full[s], x, row0_3);
+                        tma_load_2d(st + st_d1, &jd->t1, &st_full[s], x, c0);
+                        tma_load_4d(st + st_d2, &jd->t2, &st_full[s], 0, row0_2, x / 16, 0);
+                        if (++s == nst) { s = 0; ph ^= 1; }
                     }
             if (!ok)
-                for (int q = max(0, ns - NSTAGE); q < ns; ++q)
-                    for (long long i = 0; i < WAIT_LIMIT && !mbar_try_wait(&st_full[q % NSTAGE], ((q / NSTAGE) & 1)); ++i)
+                for (int q = max(0, ns - nst); q < ns; ++q)
+                    for (long long i = 0; i < WAIT_LIMIT && !mbar_try_wait(&st_full[q % nst], ((q / nst) & 1)); ++i)
                         __nanosleep(100);
         }
-    } else if (warp == WARP_MMA) {
-        // The whole warp runs the issue loop and polls the barriers together; one elected lane
-        // issues.  The tensor pipe queues only about two MMAs, so the loop is kept to a few
-        // instructions per MMA: the B descriptors move with the start address alone (bits 0-13,
-        // 16-byte units, no carry out for shared-memory addresses), the first anchor group of a
-        // sweep is peeled so that the accumulate flag is an immediate.
-        // S32 accumulate, signed int8 A and B, both K-major, M = 128, N = nmma
-        const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nmma >> 3) << 17) |
-                               ((uint32_t)(LS_ROWS >> 4) << 24);
-        const uint32_t lbo = (uint32_t)jd->span2 * 16;          // the second 16-pixel group of a digit
-        const uint64_t ddig = (uint64_t)((2 * lbo) >> 4);        // the next digit plane
-        const uint64_t desc0 = smem_desc_plain(smem_u32(smem + ST_D2), lbo) - (uint64_t)c0;  // row c0 at offset 0
-        const uint32_t accA = tmem, accB = tmem + ACC_STRIDE, accC = tmem + 2 * ACC_STRIDE;
-        const int ngr = g1 - g0;
-        int ns = 0, na = 0, ni = 0;
-        for (long b = u.b0; b < u.b1 && ok; ++b)
-            for (int sw = 0; sw < sweeps && ok; ++sw, ++ni) {
-                // the epilogue of the previous item has read the accumulators out
-                if (!mbar_wait_conv(acc_empty, (ni & 1) ^ 1, abort_flag, err, 32)) { ok = false; break; }
-                for (int sl = 0; sl < nslices(b) && ok; ++sl, ++ns) {
-                    const int s = ns % NSTAGE;
-                    if (!mbar_wait_conv(&st_full[s], (ns / NSTAGE) & 1, abort_flag, err, 33)) { ok = false; break; }
-                    const uint64_t sdesc = desc0 + (uint64_t)((s * ST_BYTES) >> 4);
-                    for (int g = 0; g < ngr; ++g, ++na) {
-                        const int ab = na % NABUF;
-                        if (!mbar_wait_conv(&ab_full[ab], (na / NABUF) & 1, abort_flag, err, 34)) { ok = false; break; }
-                        fence_after();
-                        const uint64_t q0 = sdesc + (uint64_t)sgroups[g], q1 = q0 + ddig, q2 = q1 + ddig;
-                        const uint32_t a0 = tmem + A_COL0 + ab * ABUF_COLS;
-                        if (sw == 0) {
-                            // class k = Σ_{i+j=k} Q_i·P_j into accumulator k
-                            if (sl == 0 && g == 0) {
-                                umma_i8_set(accA, a0, q0, idesc);
-                                umma_i8_set(accB, a0 + 8, q0, idesc);
-                                umma_i8_set(accC, a0 + 16, q0, idesc);
-                            } else {
-                                umma_i8_add(accA, a0, q0, idesc);
-                                umma_i8_add(accB, a0 + 8, q0, idesc);
-                                umma_i8_add(accC, a0 + 16, q0, idesc);
-                            }
-                            umma_i8_add(accB, a0, q1, idesc);
-                            umma_i8_add(accC, a0 + 8, q1, idesc);
-                            umma_i8_add(accC, a0, q2, idesc);
-                        } else {
-                            // class 3: P3·Q0 + P2·Q1 + P1·Q2; the A buffer holds P1, P2, P3
-                            if (sl == 0 && g == 0) umma_i8_set(accA, a0 + 16, q0, idesc);
-                            else umma_i8_add(accA, a0 + 16, q0, idesc);
-                            umma_i8_add(accA, a0 + 8, q1, idesc);
-                            umma_i8_add(accA, a0, q2, idesc);
-                        }
-                        umma_commit_elect(&ab_empty[ab]);
-                    }
-                    if (ok) umma_commit_elect(&st_empty[s]);
+    } else if (warp == WARP_SCALE) {
+        // scales each stage's D1 rows by 127·2^−(E1+E3) once for every row that uses them
+        const int n4 = (c1 - c0) * (SLICE / 4);
+        int s = 0, ph = 0;
+        for (long b = u.b0; b < u.b1 && ok; ++b) {
+            const float sc = ldexpf(127.f, -(jd->e1[b] + jd->e3[b]));
+            for (int i = 0; i < nslices(b) * sweeps; ++i) {
+                if (!mbar_wait_warp(&st_full[s], ph, abort_flag, err, 38)) { ok = false; break; }
+                float4 *d1 = reinterpret_cast<float4 *>(stages + s * st_bytes + jd->st_d1);
+                for (int e = lane; e < n4; e += 32) {
+                    float4 v = d1[e];
+                    v.x *= sc;
+                    v.y *= sc;
+                    v.z *= sc;
+                    v.w *= sc;
+                    d1[e] = v;
                 }
-                if (ok) umma_commit_elect(acc_full);
+                // these generic writes precede the TMA write that reuses the stage
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&st_ready[s]);
+                if (++s == nst) { s = 0; ph ^= 1; }
             }
-        if (!ok) {
-            umma_commit_elect(drain);
-            if (lane == 0)
-                for (long long i = 0; i < WAIT_LIMIT && !mbar_try_wait(drain, 0); ++i) __nanosleep(100);
-            __syncwarp();
         }
+    } else if (warp == WARP_MMA || warp == WARP_MMA2) {
+        // Two warps issue the MMAs, each into accumulators of its own (the first classes 0 and 1, the
+        // second class 2; on sweep 2 the two share class 3's sum between two accumulators), so no
+        // accumulator depends on the order of the two issuing threads.  One elected thread of each runs the
+        // whole loop: its operands are then uniform values for the compiler, which the shuffles say for
+        // those that come from memory.  The B descriptors move with the start address alone (bits 0-13,
+        // 16-byte units, no carry out for shared-memory addresses).
+        const bool second = warp == WARP_MMA2;
+        auto uni = [](int v) { return (uint32_t)__shfl_sync(0xffffffffu, v, 0); };
+        IssueState t;
+        t.ngr = uni(ngr);
+        t.nmma = uni(nmma);
+        t.nabuf = uni(nabuf);
+        t.nst = uni(nst);
+        const uint32_t lbo = uni(jd->span2) * 16;               // the second 16-pixel group of a digit
+        const uint64_t desc0 = smem_desc_plain(smem_u32(stages + uni(jd->st_d2)), lbo);
+        t.ddig = (2 * lbo) >> 4;
+        t.desc_lo = (uint32_t)desc0;
+        t.desc_hi = (uint32_t)(desc0 >> 32);
+        t.stage16 = uni(st_bytes) >> 4;
+        t.groups = smem_u32(sgroups);
+        t.flags = smem_u32(ab_flags);
+        t.bars = smem_u32(ab_empty);
+        const uint32_t tmem_u = uni((int)tmem);
+        t.acc = tmem_u + (second ? 2 * t.nmma : 0);
+        t.a_first = tmem_u + 3 * t.nmma;
+        t.ab = t.seen = t.s = t.ph = 0;
+        t.need = 4;
+        if (elect_one()) {
+            int ni = 0;
+            for (long b = u.b0; b < u.b1 && ok; ++b)
+                for (int sw = 0; sw < sweeps && ok; ++sw, ++ni) {
+                    // the epilogue of the previous item has read the accumulators out
+                    ok = mbar_wait(acc_empty, (ni & 1) ^ 1, abort_flag, err, 32);
+                    const int nsl = nslices(b);
+                    if (ok && sw == 0)
+                        ok = second ? issue_item<true, 0>(t, nsl, st_full, st_empty, abort_flag, err)
+                                    : issue_item<false, 0>(t, nsl, st_full, st_empty, abort_flag, err);
+                    else if (ok)
+                        ok = second ? issue_item<true, 1>(t, nsl, st_full, st_empty, abort_flag, err)
+                                    : issue_item<false, 1>(t, nsl, st_full, st_empty, abort_flag, err);
+                    if (ok) umma_commit_bar(smem_u32(acc_full));
+                }
+            if (!ok) {
+                uint64_t *dr = drain + (second ? 1 : 0);
+                umma_commit_bar(smem_u32(dr));
+                for (long long i = 0; i < WAIT_LIMIT && !mbar_try_wait(dr, 0); ++i) __nanosleep(100);
+            }
+        }
+        __syncwarp();
     } else {
         // ---- warps 0-15: form the A digits, then each block's epilogue ----
         const int q = warp & 3, ps = warp >> 2;
-        const int r = 32 * q + lane;                      // TMEM lane = accumulator row
-        const int a = ks > 1 ? r / nclen : 0;             // anchor slot of the row
-        const int d3 = ks > 1 ? r % nclen : r;            // lag Δ3 within the tile
-        const bool row_ok = r < mrows;
         const uint32_t lane_field = (uint32_t)(32 * q) << 16;
-        const int ngr = g1 - g0, nab1 = c1 - c0;
-        const int row0_3 = c0 - jd->nc10 + (ks > 1 ? 0 : LS_ROWS * u.t3);  // channel of staged D3 row 0
-        int ns = 0, na = 0, ni = 0;
-        // The 16 formers are four sets of four: set ps forms anchor groups ps, ps + 4, … of each
-        // slice, and within a set warp q fills TMEM lanes 32q .. 32q+31 of the group's A buffer
-        // with all 32 pixels (four 8-pixel chunks, one tcgen05.st.x8 per digit plane), so the
-        // per-group work (addresses, barrier wait, TMEM hand-off) is spread over 32 pixels.  A
-        // lane whose row has no data (past the tile or past the anchor block) reads a zeroed row,
-        // so its digits come out zero with no per-digit select; D3 channels outside [0, nc) arrive
-        // as zero rows from the TMA bounds fill, and a warp whose rows all lie there stores zero
-        // digits without the arithmetic.
-        auto form_slice = [&](auto ndc, const unsigned char *st) {
+        const int nab1 = c1 - c0;
+        const uint32_t stage0 = smem_u32(stages), st_d1 = (uint32_t)jd->st_d1;
+        const uint32_t flag0 = smem_u32(ab_flags), group0 = smem_u32(sgroups) + 12;
+        // TMEM lane 32q + 8j + i holds accumulator row 8·(4j + q) + 4·(i & 1) + i / 2.  The 8-row blocks
+        // go round the four quarters of the lanes, so that the blocks an anchor's window leaves empty (a
+        // quarter to half of them) come off all four SM partitions alike; and the two lanes that one
+        // eight-thread phase of a shared load reads (below) hold rows four apart, whose 128-byte swizzles
+        // differ in the half of the row, so the phase is free of bank conflicts.
+        auto row_of = [](int L) { return 8 * ((L >> 1 & 12) | L >> 5) + ((L & 1) << 2 | (L >> 1 & 3)); };
+        // The 16 formers are four sets of four: set ps forms every fourth anchor group of the
+        // item's sequence (slices, groups within a slice), and within a set warp q fills TMEM lanes
+        // 32q .. 32q+31 of the group's A buffer with all 32 pixels, so the per-group work
+        // (addresses, waits, TMEM hand-off) is spread over 32 pixels.  A thread forms four rows
+        // (lanes t/4 + 8j, one 8-row block each) of two 4-pixel words each (words t%4 and 4 + t%4), so its
+        // two D1 words serve every row of an anchor slot.  A block without a row in range stores zero
+        // digits without the arithmetic.  The first lanes' digits are formed before the buffer is waited for.  Rows past a slot's lags hold digits of whatever was read: their
+        // accumulator rows are never read out.  D3 channels outside [0, nc) arrive as zero rows from the TMA
+        // bounds fill.
+        const uint32_t c4 = (lane & 3) << 4;
+        // 16 × (D3 row less the group's first row) and 16 × anchor slot of the thread's rows
+        uint32_t roff[4], slot[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int r = row_of(32 * q + 8 * j + (lane >> 2));
+            slot[j] = ks > 1 ? 16 * (r / rs) : 0;
+            roff[j] = ks > 1 ? slot[j] + 16 * (r % rs) : 16 * r;
+        }
+        int s = 0, ph = 0, ni = 0, ab = ps % nabuf;
+        int g = ps;               // next group of this set, counted from the current slice's first
+        uint32_t abph = 1 ^ (ps / nabuf & 1);  // parity to wait for on ab_empty[ab]
+        auto form_slice = [&](auto ndc, auto onec) {
             constexpr int ND = decltype(ndc)::value;
-            constexpr int D0 = ND - 3;  // sweep 2 stores product digits 1-3
-            for (int g = ps; g < ngr && ok; g += NSET) {
-                const int n = na + g;  // the group's place in the MMA warp's order
-                if (!mbar_wait_warp(&ab_empty[n % NABUF], ((n / NABUF) & 1) ^ 1, abort_flag, err, 36)) {
-                    ok = false;
-                    break;
+            constexpr int D0 = ND - 3;                    // sweep 2 stores product digits 1-3
+            constexpr bool ONE = decltype(onec)::value;   // one anchor slot
+            const uint32_t st = stage0 + (uint32_t)(s * st_bytes);
+            for (; g < ngr; g += NSET) {
+                uint32_t word;
+                asm volatile("ld.shared.b32 %0, [%1];" : "=r"(word) : "r"(group0 + 16 * g));
+                word = __shfl_sync(0xffffffffu, word, 0);
+                const uint32_t row = word & 0xffffu, blocks = word >> (16 + q);  // 16 × first row, live blocks
+                const uint32_t col = a_col0 + lane_field + ab * ABUF_COLS;
+                // 16-byte chunk c of a 128-byte-swizzled row lies at chunk c ^ (row & 7)
+                auto chunk_of = [&](uint32_t r16) { return st + 8 * r16 + ((r16 & 0x70u) ^ c4); };
+                float4 v1[2];
+                uint32_t a3[2] = {0, 0};  // words t%4 and 4 + t%4 of the D3 row
+                if constexpr (ONE) {
+                    a3[0] = chunk_of(row + roff[0]);
+                    a3[1] = a3[0] ^ 64;
+                    const uint32_t a1 = st_d1 + chunk_of(row);
+                    v1[0] = lds128(a1);
+                    v1[1] = lds128(a1 ^ 64);
                 }
-                const int p1 = sgroups[g] + a;
-                const int rho = p1 - c0 + d3;  // staged D3 row of this lane
-                const bool valid = row_ok && p1 < c1;
-                const int p3 = row0_3 + rho;  // D3 channel of this lane's row
-                // two halves of 16 pixels: 12 digit words stay live until their tcgen05.wait::st
-                // (the 18 warps leave ~96 registers a thread)
-                const bool live = __any_sync(0xffffffffu, valid && p3 >= 0 && p3 < nc);
-                const unsigned char *row3 = valid ? st + ST_D3 + rho * 128 : zero_row;
-                // the D1 row, already scaled by 127·2^−(E1+E3) for this block
-                const float4 *row1 = reinterpret_cast<const float4 *>(st + ST_D1 + min(p1 - c0, nab1 - 1) * 128);
-                const uint32_t col = tmem + lane_field + A_COL0 + (n % NABUF) * ABUF_COLS;
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
+                for (int half = 0; half < 2; ++half) {  // TMEM lanes 16·half .. +15 of the warp's 32
                     uint32_t w[3][4];
-                    if (live) {
 #pragma unroll
-                        for (int cc = 0; cc < 2; ++cc) {
-                            const int c = 2 * half + cc;
-                            const float4 x0 = *reinterpret_cast<const float4 *>(row3 + (((2 * c) ^ (rho & 7)) << 4));
-                            const float4 x1 =
-                                *reinterpret_cast<const float4 *>(row3 + (((2 * c + 1) ^ (rho & 7)) << 4));
-                            const float4 u0 = row1[2 * c], u1 = row1[2 * c + 1];
-                            {  // pixels 0-3 of the chunk -> word 2cc of each digit plane
+                    for (int jj = 0; jj < 2; ++jj) {
+                        const int j = 2 * half + jj;
+                        if (blocks >> (4 * j) & 1) {
+                            if constexpr (!ONE) {
+                                a3[0] = chunk_of(row + roff[j]);
+                                a3[1] = a3[0] ^ 64;
+                                const uint32_t a1 = st_d1 + chunk_of(row + slot[j]);
+                                v1[0] = lds128(a1);
+                                v1[1] = lds128(a1 ^ 64);
+                            }
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                const float4 x = lds128(a3[h] + (ONE ? 4096 * j : 0));
                                 float2 ya[4], yb[4];
-                                digits254x2<ND>(make_float2(u0.x, u0.y), make_float2(x0.x, x0.y), ya);
-                                digits254x2<ND>(make_float2(u0.z, u0.w), make_float2(x0.z, x0.w), yb);
+                                digits254x2<ND>(make_float2(v1[h].x, v1[h].y), make_float2(x.x, x.y), ya);
+                                digits254x2<ND>(make_float2(v1[h].z, v1[h].w), make_float2(x.z, x.w), yb);
 #pragma unroll
                                 for (int dd = 0; dd < 3; ++dd)
-                                    w[dd][2 * cc] =
+                                    w[dd][2 * h + jj] =
                                         pack_low_bytes(ya[dd + D0].x, ya[dd + D0].y, yb[dd + D0].x, yb[dd + D0].y);
                             }
-                            {  // pixels 4-7 -> word 2cc + 1
-                                float2 yc[4], yd[4];
-                                digits254x2<ND>(make_float2(u1.x, u1.y), make_float2(x1.x, x1.y), yc);
-                                digits254x2<ND>(make_float2(u1.z, u1.w), make_float2(x1.z, x1.w), yd);
+                        } else {
 #pragma unroll
-                                for (int dd = 0; dd < 3; ++dd)
-                                    w[dd][2 * cc + 1] =
-                                        pack_low_bytes(yc[dd + D0].x, yc[dd + D0].y, yd[dd + D0].x, yd[dd + D0].y);
-                            }
+                            for (int dd = 0; dd < 3; ++dd) w[dd][jj] = w[dd][2 + jj] = 0u;
                         }
-                    } else {
-#pragma unroll
-                        for (int dd = 0; dd < 3; ++dd)
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) w[dd][e] = 0u;
                     }
-                    // pixels 16·half .. +15 = columns 4·half .. +3 of each digit plane
+                    if (half == 0) {
+                        if (!mbar_wait_conv(&ab_empty[ab], abph, abort_flag, err, 36)) { ok = false; return; }
+                        fence_after();
+                    }
 #pragma unroll
-                    for (int dd = 0; dd < 3; ++dd) tmem_st4(col + 8 * dd + 4 * half, w[dd]);
-                    // tcgen05.st reads its source registers asynchronously: wait before they change
-                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    for (int dd = 0; dd < 3; ++dd) tmem_st16x8(col + ((uint32_t)(16 * half) << 16) + 8 * dd, w[dd]);
                 }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&ab_full[n % NABUF]);
+                if (lane == 0) count_add(flag0 + ab * 4);
+                ab += NSET;
+                while (ab >= nabuf) { ab -= nabuf; abph ^= 1; }
             }
-            na += ngr;
+            g -= ngr;
         };
         for (long b = u.b0; b < u.b1 && ok; ++b) {
-            const int E13 = jd->e1[b] + jd->e3[b];
-            const float sc = ldexpf(127.f, -E13);
+            const int E = jd->e1[b] + jd->e3[b] + jd->e2[b];
             for (int sw = 0; sw < sweeps && ok; ++sw, ++ni) {
-                for (int sl = 0; sl < nslices(b) && ok; ++sl, ++ns) {
-                    const int s = ns % NSTAGE;
-                    if (!mbar_wait_warp(&st_full[s], (ns / NSTAGE) & 1, abort_flag, err, 35)) { ok = false; break; }
-                    unsigned char *st = smem + s * ST_BYTES;
-                    // scale the staged D1 rows once for every row that uses them (the formers alone read them)
-                    float *d1 = reinterpret_cast<float *>(st + ST_D1);
-                    for (int e = tid; e < nab1 * SLICE; e += NFORM * 32) d1[e] *= sc;
-                    asm volatile("bar.sync 1, %0;" ::"n"(NFORM * 32) : "memory");
-                    if (sw == 0) form_slice(std::integral_constant<int, 3>(), st);
-                    else form_slice(std::integral_constant<int, 4>(), st);
+                for (int sl = 0; sl < nslices(b); ++sl) {
+                    if (!mbar_wait_conv(&st_ready[s], ph, abort_flag, err, 35)) { ok = false; break; }
+                    if (ks == 1) {
+                        if (sw == 0) form_slice(std::integral_constant<int, 3>(), std::true_type());
+                        else form_slice(std::integral_constant<int, 4>(), std::true_type());
+                    } else {
+                        if (sw == 0) form_slice(std::integral_constant<int, 3>(), std::false_type());
+                        else form_slice(std::integral_constant<int, 4>(), std::false_type());
+                    }
+                    if (!ok) break;
                     __syncwarp();
-                    if (ok && lane == 0) mbar_arrive(&st_empty[s]);
+                    if (lane == 0) mbar_arrive(&st_empty[s]);
+                    if (++s == nst) { s = 0; ph ^= 1; }
                 }
                 if (!ok) break;
                 // ---- epilogue: int32 class accumulators → FP64, added into the unit's partial tile ----
                 if (!mbar_wait_warp(acc_full, ni & 1, abort_flag, err, 37)) { ok = false; break; }
                 fence_after();
-                const int E = E13 + jd->e2[b];
                 const double scale = sw == 0 ? ldexp(1.0, E) * (1.0 / (16129.0 * 64516.0))
                                              : ldexp(1.0, E) * (1.0 / (16129.0 * 16387064.0));
                 const bool first = b == u.b0 && sw == 0;
-                for (int cb = 8 * ps; cb < nmma; cb += 32) {
+                // this lane's accumulator row and anchor slot
+                const int r = row_of(32 * q + lane), a = ks > 1 ? r / rs : 0;
+                const bool row_ok = ks > 1 ? r < mrows && r - a * rs < nclen : r < mrows;
+                for (int cb = 8 * ps; cb < nmma; cb += 8 * NSET) {
                     uint32_t v0[8], v1[8], v2[8];
                     tmem_ld8(tmem + lane_field + cb, v0);
-                    if (sw == 0) {
-                        tmem_ld8(tmem + lane_field + ACC_STRIDE + cb, v1);
-                        tmem_ld8(tmem + lane_field + 2 * ACC_STRIDE + cb, v2);
-                    }
+                    if (sw == 0) tmem_ld8(tmem + lane_field + nmma + cb, v1);
+                    tmem_ld8(tmem + lane_field + 2 * nmma + cb, v2);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     if (!row_ok) continue;
 #pragma unroll
@@ -464,7 +660,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                         if (colx < 0 || colx >= ncols) continue;
                         const long long V = sw == 0 ? (long long)(int)v0[e] * 64516LL + (long long)(int)v1[e] * 254LL +
                                                           (long long)(int)v2[e]
-                                                    : (long long)(int)v0[e];
+                                                    : (long long)(int)v0[e] + (long long)(int)v2[e];
                         double *o = out + (long)colx * LS_ROWS + r;
                         const double val = (double)V * scale;
                         *o = first ? val : *o + val;
@@ -484,8 +680,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
     }
 }
-
-constexpr size_t SMEM_BYTES = 1024 + (size_t)NSTAGE * ST_BYTES + 256 + sizeof(int) * LS_SPAN + 128;
 
 typedef CUresult (*EncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                 const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
@@ -588,7 +782,7 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
             const cuuint64_t fstr[1] = {(cuuint64_t)jb.kp * 4};
             const cuuint32_t box3[2] = {SLICE, (cuuint32_t)x.span3}, box1[2] = {SLICE, (cuuint32_t)s.AB};
             if ((rc = encode(c, &x.t3, f32, 2, jb.m3.f32, fdims, fstr, box3, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
-            if ((rc = encode(c, &x.t1, f32, 2, jb.m1.f32, fdims, fstr, box1, CU_TENSOR_MAP_SWIZZLE_NONE))) return rc;
+            if ((rc = encode(c, &x.t1, f32, 2, jb.m1.f32, fdims, fstr, box1, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
             const cuuint64_t ddims[4] = {16, (cuuint64_t)jb.nc, (cuuint64_t)(jb.kp / 16), 3};
             const cuuint64_t dstr[3] = {16, (cuuint64_t)jb.nc * 16, (cuuint64_t)jb.nc * jb.kp};
             const cuuint32_t box2[4] = {16, (cuuint32_t)x.span2, 2, 3};
@@ -603,16 +797,24 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
             x.nc10 = jb.nc10;
             x.nclen = s.nclen;
             x.ks = s.k;
+            x.rs = s.rs;
             x.AB = s.AB;
             x.T = s.T;
             x.sweeps = jb.mask_pass ? 2 : 1;
             x.tx_bytes = (uint32_t)(x.span3 * 128 + s.AB * 128 + 3 * 2 * x.span2 * 16);
+            // whole 8-row swizzle atoms for the fp32 rows; every part starts on a 1024-byte boundary.  The
+            // formers read a slot's whole 8-row blocks (all LS_ROWS rows with one slot) from every anchor on,
+            // past the tile's rows too.
+            x.st_d1 = (s.AB - 1 + (s.k > 1 ? s.rs : LS_ROWS) + 7) / 8 * 1024;
+            x.st_d2 = x.st_d1 + (s.AB + 7) / 8 * 1024;
+            x.st_bytes = x.st_d2 + (3 * 2 * x.span2 * 16 + 1023) / 1024 * 1024;
+            x.nst = std::min(NSTAGE_MAX, SMEM_STAGES / x.st_bytes);
             std::copy(p.groups.begin(), p.groups.end(), hg + gpos);
             for (size_t q = 0; q < p.group_off.size(); ++q) ho[opos + q] = p.group_off[q];
             gpos += p.groups.size();
             opos += p.group_off.size();
             red.push_back(LsReduceJob{(const double *)c->partial.p + p.unit_base * LS_ROWS * LS_ROWS, jb.lag_out,
-                                      s.nclen, s.k, s.T, s.nab, s.V});
+                                      s.nclen, s.k, s.rs, s.T, s.nab, s.V});
         }
         std::copy(units.begin(), units.end(), (LsUnit *)(h + off_u));
         if ((rc = cuda_check(c, cudaMemcpyAsync(d, h, stage_b, cudaMemcpyHostToDevice, c->stream), "job list upload")))

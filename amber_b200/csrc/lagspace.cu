@@ -30,7 +30,7 @@ __global__ void ls_reduce_kernel(const LsReduceJob *__restrict__ jobs)
     if (j.k > 1) {
         for (int u = 0; u < j.nab * j.V; ++u) {
             const double *p = j.partial + u * TILE + (long)d2 * LS_ROWS;
-            for (int a = 0; a < j.k; ++a) add(p[a * j.nclen + d3]);
+            for (int a = 0; a < j.k; ++a) add(p[a * j.rs + d3]);
         }
     } else {
         const int t2 = d2 / LS_ROWS, c = d2 % LS_ROWS, t3 = d3 / LS_ROWS, r = d3 % LS_ROWS;
@@ -42,7 +42,7 @@ __global__ void ls_reduce_kernel(const LsReduceJob *__restrict__ jobs)
 
 }  // namespace
 
-int LsShape::rows(int t3) const { return k > 1 ? k * nclen : std::min(LS_ROWS, nclen - LS_ROWS * t3); }
+int LsShape::rows(int t3) const { return k > 1 ? k * rs : std::min(LS_ROWS, nclen - LS_ROWS * t3); }
 int LsShape::cols(int t2) const
 {
     return k > 1 ? round16(nclen + k - 1) : round16(std::min(LS_ROWS, nclen - LS_ROWS * t2));
@@ -55,7 +55,8 @@ LsShape ls_shape(int nc, int nc10, long k_px, int sms, long min_bpu, long force_
     s.nc = nc;
     s.nc10 = nc10;
     s.nclen = 2 * nc10 + 1;
-    s.k = s.nclen <= LS_ROWS / 2 ? LS_ROWS / s.nclen : 1;
+    s.rs = (s.nclen + 7) / 8 * 8;
+    s.k = s.rs <= LS_ROWS / 2 ? LS_ROWS / s.rs : 1;
     s.T = s.k > 1 ? 1 : (s.nclen + LS_ROWS - 1) / LS_ROWS;
     // Staged rows of one unit: D3 spans AB + rows − 1 channels and the D2 window AB + N − 1;
     // both must fit one TMA box (LS_SPAN rows).  An anchor block also holds at most 128 anchor

@@ -17,10 +17,11 @@
 // more than once) weight the operands; rows outside [0, nc) are zero.
 //
 // Tiles.  Accumulator rows are Δ3 (128 per tile), columns Δ2 (N per tile).
-// Small lag windows (nclen ≤ 64) put k = ⌊128/nclen⌋ consecutive anchors into
-// one tile: row r = a·nclen + Δ3 holds anchor slot a, and B is the window of
-// the first anchor widened to N = nclen + k − 1 rows, so slot a's lag is
-// Δ2 = column − a.  Large windows (nclen > 128) use ⌈nclen/128⌉² tile pairs.
+// Small lag windows (nclen ≤ 64) put k = ⌊128/rs⌋ consecutive anchors into one
+// tile, rs being nclen rounded up to a multiple of 8 (so that an 8-row block
+// belongs to one anchor): row r = a·rs + Δ3 holds anchor slot a, and B is the
+// window of the first anchor widened to N = nclen + k − 1 rows, so slot a's lag
+// is Δ2 = column − a.  Large windows (nclen > 128) use ⌈nclen/128⌉² tile pairs.
 //
 // Work units.  The pixels are cut into blocks of LS_BLOCK; a unit is a tile
 // pair × an anchor block × a run of consecutive pixel blocks, run by one CTA,
@@ -44,6 +45,7 @@ constexpr int LS_SPAN = 256;   // most channel rows one unit stages (a TMA box h
 struct LsShape {
     int nc, nc10, nclen;
     int k;        // anchor slots per tile (1 unless nclen ≤ 64)
+    int rs;       // rows from one anchor slot to the next: nclen rounded up to whole 8-row blocks
     int T;        // tiles per lag axis
     int AB, nab;  // anchor-block width in channels, number of anchor blocks
     long nblk;    // pixel blocks
@@ -88,7 +90,7 @@ void ls_units(const LsJobPlan &p, int job, std::vector<LsUnit> &out);
 struct LsReduceJob {
     const double *partial;  // the job's partial tiles [units][LS_ROWS][LS_ROWS]
     double *lag;            // FP64 lag array [nclen][nclen], row Δ2, column Δ3
-    int nclen, k, T, nab, V;
+    int nclen, k, rs, T, nab, V;
 };
 // lag = Σ over units (and slots) of the partial tiles, compensated, fixed order; one launch for
 // every job of a contraction launch.  The descriptors are copied into the context's job staging.
