@@ -4,10 +4,14 @@
 // FP64 triple sum that gives calCR's normaliser (amber_funcs.c:451-457).
 //
 // The contraction is the lag-space GEMM of lagspace.cuh: per unit (a tile pair,
-// an anchor block and a run of pixel blocks) one CTA of 8 warps holds a 128 × 128
-// FP64 accumulator tile in registers, 16 warps each holding a 32 × 32 block as
-// 2 × 4 fragments of the FP64 tensor-core MMA mma.sync m16n8k8 (1024 FMAs per
-// instruction; the m8n8k4 shape reaches only about half the FP64 tensor rate).  Per stage of 16
+// an anchor block and a run of pixel blocks) one CTA of 16 warps holds a 128 × 128
+// FP64 accumulator tile in registers, each warp two 16-row by four 8-column
+// fragments of the FP64 tensor-core MMA mma.sync m16n8k8 (1024 FMAs per
+// instruction; the m8n8k4 shape reaches only about half the FP64 tensor rate).
+// Fragments outside an anchor's channel range are skipped: the kernel is bound by
+// the DMMA pipe (84 % busy with every fragment computed), and at nc10 = nc − 1 three
+// quarters of the fragments are empty, at nc10 = nc/2 − 1 two fifths (46 triangles of
+// 32 channels: 66.6 → 28.9 ms of kernel time).  Per stage of 16
 // pixels the CTA copies the channel rows its anchors touch — w·D1 of the anchor
 // block, w·D3 and w·D2 of the spans their windows cover — into shared memory
 // once (transposed, [pixel][channel]); then, for every anchor group, it forms
@@ -67,7 +71,11 @@ __global__ void __launch_bounds__(F_NT, 1) ls_fp64_kernel(const F64Desc *__restr
     const LsUnit u = units[blockIdx.x];
     const F64Desc j = jobs[u.job];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int wm = warp >> 2, wn = warp & 3;   // warp tile: rows 32·wm .., columns 32·wn ..
+    // Warp fragments: row fragments wm and wm + 4 (16 rows each), column fragments wc, wc + 4, .. (8 columns
+    // each).  An anchor's live rows and columns are contiguous ranges, so fragments are dealt round the
+    // warps, and the column class is shifted by wm so that the four warps of one SM partition (equal
+    // warp mod 4) hold all four classes: every partition gets the same share of whatever range is live.
+    const int wm = warp >> 2, wc = (warp + wm) & 3;
     const int gq = lane >> 2, tq = lane & 3;   // fragment row / column group, k index
     const int ks = j.ks, nclen = j.nclen, nc = j.nc;
     const int c0 = u.ab * j.AB, c1 = min(nc, c0 + j.AB), nab1 = c1 - c0;
@@ -77,7 +85,34 @@ __global__ void __launch_bounds__(F_NT, 1) ls_fp64_kernel(const F64Desc *__restr
     const int row0_2 = c0 - j.nc10 + (ks > 1 ? 0 : LS_ROWS * u.t2);  // channel of staged D2 row 0
     const int span3 = nab1 + (ks > 1 ? nclen : mrows) - 1;
     const int span2 = nab1 + ncols - 1;
-    const int g0 = j.group_off[u.ab], g1 = j.group_off[u.ab + 1];
+    const int toff3 = ks > 1 ? 0 : LS_ROWS * u.t3, toff2 = ks > 1 ? 0 : LS_ROWS * u.t2;
+    // The unit's anchor groups {first channel, live column fragments (bits 0-15) and row fragments (bits
+    // 16-23)}: fragments whose D2 or D3 channels all lie outside [0, nc) add only zeros and are skipped, and
+    // a group without a live fragment (a corner tile of a wide window) is dropped.
+    __shared__ uint2 sgroups[LS_SPAN];
+    __shared__ int ngroups_s;
+    if (warp == 0) {
+        const int g0 = j.group_off[u.ab], g1 = j.group_off[u.ab + 1];
+        int n = 0;
+        for (int gb = g0; gb < g1; gb += 32) {
+            const int pb = gb + lane < g1 ? j.groups[gb + lane] : 0;
+            const int w2 = pb - j.nc10 + toff2, w3 = pb - j.nc10 + toff3;  // channels of the first column and row
+            const int lo = max(0, -w2), hi = min(ncols, nc - w2);
+            uint32_t m = 0, rows = 0;
+            if (lo < hi) m = (0xffffu << (lo / 8)) & (0xffffu >> (15 - (hi - 1) / 8));
+            for (int a = 0; a < ks && pb + a < c1; ++a) {
+                const int ra = max(0, -(w3 + a)), rb = min(ks > 1 ? nclen : mrows, nc - (w3 + a));  // its lags in range
+                if (ra < rb) rows |= (0xffu << ((a * j.rs + ra) / 16)) & (0xffu >> (7 - (a * j.rs + rb - 1) / 16));
+            }
+            const bool keep = gb + lane < g1 && m && rows;
+            const unsigned kept = __ballot_sync(0xffffffffu, keep);
+            if (keep) sgroups[n + __popc(kept & ((1u << lane) - 1u))] = make_uint2((uint32_t)pb, m | rows << 16);
+            n += __popc(kept);
+        }
+        if (lane == 0) ngroups_s = n;
+    }
+    __syncthreads();
+    const int ngr = ngroups_s;
     // the A row this thread forms (pixels tid/128 + 4i), its anchor slot and lag
     const int ar = tid & (LS_ROWS - 1), ax = tid >> 7;
     const int aslot = ks > 1 ? ar / j.rs : 0, ad3 = ks > 1 ? ar % j.rs : ar;
@@ -110,7 +145,7 @@ __global__ void __launch_bounds__(F_NT, 1) ls_fp64_kernel(const F64Desc *__restr
     };
 
     int buf = 0;
-    for (long b = u.b0; b < u.b1; ++b) {
+    for (long b = u.b0; b < u.b1 && ngr > 0; ++b) {
         const long xb = b * LS_BLOCK;
         for (long x0 = xb; x0 < min(j.k, xb + LS_BLOCK); x0 += F_KX) {
             __syncthreads();  // every reader of the previous stage is done
@@ -118,8 +153,11 @@ __global__ void __launch_bounds__(F_NT, 1) ls_fp64_kernel(const F64Desc *__restr
             stage(st3, F_S3, j.m3, row0_3, span3, x0);
             stage(st2, F_S2, j.m2, row0_2, span2, x0);
             __syncthreads();
-            for (int g = g0; g < g1; ++g) {
-                const int pb = j.groups[g];
+            for (int g = 0; g < ngr; ++g) {
+                const int pb = (int)sgroups[g].x;
+                const uint32_t live = sgroups[g].y;
+                const bool row0 = live >> (16 + wm) & 1, row1 = live >> (20 + wm) & 1;
+                const uint32_t cols = row0 || row1 ? live >> wc & 0x1111u : 0u;
                 // A[x][r] = D1[p1, x] · D3[p1 − nc10 + Δ3, x] for slot a and lag Δ3 of row r.  A[buf] was
                 // last read two groups ago, before the barrier that ended the previous formation.
                 double *A = As + buf * (F_KX * F_SA);
@@ -131,28 +169,27 @@ __global__ void __launch_bounds__(F_NT, 1) ls_fp64_kernel(const F64Desc *__restr
                     A[xx * F_SA + ar] = ok ? st1[xx * F_S1 + (p1 - c0)] * st3[xx * F_S3 + (p1 - c0) + ad3] : 0.0;
                 }
                 __syncthreads();
-                const double *Aw = A + 32 * wm + gq;
-                const double *Bw = st2 + (pb - c0) + 32 * wn + gq;
+                const double *Aw = A + 16 * wm + gq;
+                const double *Bw = st2 + (pb - c0) + 8 * wc + gq;
 #pragma unroll
                 for (int k8 = 0; k8 < F_KX / 8; ++k8) {
+                    if (!cols) break;
                     const int xx = 8 * k8 + tq;
-                    double a[2][4], bv[4][2];
+                    double a[2][4];
 #pragma unroll
                     for (int mt = 0; mt < 2; ++mt) {
-                        a[mt][0] = Aw[xx * F_SA + 16 * mt];
-                        a[mt][1] = Aw[xx * F_SA + 16 * mt + 8];
-                        a[mt][2] = Aw[(xx + 4) * F_SA + 16 * mt];
-                        a[mt][3] = Aw[(xx + 4) * F_SA + 16 * mt + 8];
+                        a[mt][0] = Aw[xx * F_SA + 64 * mt];
+                        a[mt][1] = Aw[xx * F_SA + 64 * mt + 8];
+                        a[mt][2] = Aw[(xx + 4) * F_SA + 64 * mt];
+                        a[mt][3] = Aw[(xx + 4) * F_SA + 64 * mt + 8];
                     }
 #pragma unroll
                     for (int nt = 0; nt < 4; ++nt) {
-                        bv[nt][0] = Bw[xx * F_S2 + 8 * nt];
-                        bv[nt][1] = Bw[(xx + 4) * F_S2 + 8 * nt];
+                        if (!(cols >> (4 * nt) & 1)) continue;
+                        const double bv[2] = {Bw[xx * F_S2 + 32 * nt], Bw[(xx + 4) * F_S2 + 32 * nt]};
+                        if (row0) dmma(acc[0][nt], a[0], bv);
+                        if (row1) dmma(acc[1][nt], a[1], bv);
                     }
-#pragma unroll
-                    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-                        for (int nt = 0; nt < 4; ++nt) dmma(acc[mt][nt], a[mt], bv[nt]);
                 }
                 buf ^= 1;
             }
@@ -165,14 +202,14 @@ __global__ void __launch_bounds__(F_NT, 1) ls_fp64_kernel(const F64Desc *__restr
     for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
         for (int hr = 0; hr < 2; ++hr) {
-            const int r = 32 * wm + 16 * mt + 8 * hr + gq;
+            const int r = 16 * wm + 64 * mt + 8 * hr + gq;
             if (r >= mrows) continue;
             const int a = ks > 1 ? r / j.rs : 0;
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const int col = 32 * wn + 8 * nt + 2 * tq + h - a;
+                    const int col = 8 * wc + 32 * nt + 2 * tq + h - a;
                     if (col >= 0 && col < lagc) out[(long)col * LS_ROWS + r] = acc[mt][nt][2 * hr + h];
                 }
         }
