@@ -293,6 +293,9 @@ int run_next_batch(amber_cuda_ctx *c, RunState &st, std::vector<I8Job> *jobs)
     // The next batch of the group: triangles whose ring union fits the budget.
     size_t spare = c->budget > c->held ? c->budget - c->held : 0;
     spare += c->maps_d.bytes + c->maps_i.bytes + c->y.bytes;
+    // the partial tiles of the last contraction give way to maps: the mixed path's reserve below covers
+    // them, the FP64 path frees them when the maps need the room and takes what is left afterwards
+    if (!c->contracts_elsewhere) spare += c->partial.bytes;
     // keep room for the mixed-precision contraction's partial tiles when they live in this context
     const size_t reserve = ((size_t)64 << 20) +
                            (prec == AMBER_PREC_MIXED && !c->contracts_elsewhere ? contract_partial_cap(c) : 0);
@@ -323,6 +326,13 @@ int run_next_batch(amber_cuda_ctx *c, RunState &st, std::vector<I8Job> *jobs)
     }
     ms.nslots = (int)ms.ring_of_slot.size();
     const size_t nvals = (size_t)ms.nslots * c->nc * kp;
+    if (prec == AMBER_PREC_FP64) {
+        const size_t other = c->held - c->maps_d.bytes - c->maps_i.bytes - c->y.bytes;
+        if (other + reserve + map_slot_bytes(prec, g.ng, c->nc, want_v2) * ms.nslots > c->budget) {
+            if ((rc = cuda_check(c, cudaStreamSynchronize(c->stream), "partial lag tiles"))) return rc;
+            release(c, c->partial);
+        }
+    }
     if ((rc = ensure(c, c->maps_d, per_slot * ms.nslots, "ring maps"))) return rc;
     if (want_v2 && (rc = ensure(c, c->maps_i, per_slot * ms.nslots, "ring mask maps"))) return rc;
     // carve one map set (D or I) out of its buffer

@@ -329,7 +329,12 @@ int contract_fp64_jobs(amber_cuda_ctx *c, const std::vector<F64Job> &jobs)
         return AMBER_OK;
     }
     constexpr size_t TILE_B = sizeof(double) * LS_ROWS * LS_ROWS;
-    const size_t pcap = std::max<size_t>((size_t)256 << 20, contract_partial_cap(c));
+    // partial tiles of one launch: no more than the context's budget leaves beside its maps (less a margin
+    // for the job lists); a job too large for that on its own takes longer runs of blocks per unit
+    const size_t room = (c->budget > c->held ? c->budget - c->held : 0) + c->partial.bytes, margin = (size_t)8 << 20;
+    const size_t pcap = std::min(std::max<size_t>((size_t)256 << 20, contract_partial_cap(c)),
+                                 room > margin ? room - margin : 0);
+    const long tile_cap = std::max<long>(1, (long)(pcap / TILE_B));
     size_t j0 = 0;
     while (j0 < jobs.size()) {
         // plan as many jobs as their partial tiles allow in one launch
@@ -338,8 +343,12 @@ int contract_fp64_jobs(amber_cuda_ctx *c, const std::vector<F64Job> &jobs)
         size_t j1 = j0;
         for (; j1 < jobs.size(); ++j1) {
             LsJobPlan p;
-            ls_plan_job(p, (int)c->nc, c->nc10, jobs[j1].k, c->weight, c->num_sms, 8, ls_force_bpu(c->chunk_px));
-            if (j1 > j0 && (size_t)(tiles + p.s.units()) * TILE_B > pcap) break;
+            ls_plan_job(p, (int)c->nc, c->nc10, jobs[j1].k, c->weight, c->num_sms, 1, ls_force_bpu(c->chunk_px));
+            if (j1 > j0 && tiles + p.s.units() > tile_cap) break;
+            if (p.s.units() > tile_cap && c->chunk_px <= 0) {
+                const long runs = std::max<long>(1, tile_cap / (p.s.units() / p.s.V));
+                ls_plan_job(p, (int)c->nc, c->nc10, jobs[j1].k, c->weight, c->num_sms, 1, (p.s.nblk + runs - 1) / runs);
+            }
             p.unit_base = tiles;
             tiles += p.s.units();
             plans.push_back(std::move(p));

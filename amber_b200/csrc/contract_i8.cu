@@ -92,6 +92,7 @@ constexpr int TMEM_COLS = 512;
 constexpr int NSET = NFORM / 4;              // former sets: each anchor group is formed by one set of 4 warps
 constexpr int ABUF_COLS = 24;                // 3 digits × 8 columns (32 int8 per row per digit)
 constexpr int NABUF_MAX = 8;                 // A buffers: as many as TMEM holds beside the accumulators
+constexpr long MIN_GROUPS = 5;                // least work of a unit (lagspace.cuh): ~10 µs
 constexpr int NSTAGE_MAX = 8;                // stages: as many as shared memory holds
 static_assert(3 * LS_ROWS + 5 * ABUF_COLS <= TMEM_COLS, "TMEM: five A buffers beside the widest accumulators");
 
@@ -522,7 +523,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         // ---- warps 0-15: form the A digits, then each block's epilogue ----
         const int q = warp & 3, ps = warp >> 2;
         const uint32_t lane_field = (uint32_t)(32 * q) << 16;
-        const int nab1 = c1 - c0;
         const uint32_t stage0 = smem_u32(stages), st_d1 = (uint32_t)jd->st_d1;
         const uint32_t flag0 = smem_u32(ab_flags), group0 = smem_u32(sgroups) + 12;
         // TMEM lane 32q + 8j + i holds accumulator row 8·(4j + q) + 4·(i & 1) + i / 2.  The 8-row blocks
@@ -730,7 +730,7 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
         for (; j1 < jobs.size(); ++j1) {
             const I8Job &jb = jobs[j1];
             LsJobPlan p;
-            ls_plan_job(p, jb.nc, jb.nc10, jb.k, *jb.weight, c->num_sms, 8, ls_force_bpu(c->chunk_px));
+            ls_plan_job(p, jb.nc, jb.nc10, jb.k, *jb.weight, c->num_sms, MIN_GROUPS, ls_force_bpu(c->chunk_px));
             if (j1 > j0 && (size_t)(tiles + p.s.units()) * TILE_B > pcap) break;
             p.unit_base = tiles;
             tiles += p.s.units();

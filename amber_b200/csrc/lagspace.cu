@@ -11,15 +11,20 @@ namespace {
 int round16(int n) { return (n + 15) / 16 * 16; }
 
 // lag[Δ2·nclen + Δ3] = Σ over the job's units (anchor blocks, then units of the block, then
-// slots) of the partial tiles, TwoSum-compensated, in that fixed order.  Partial tiles are
-// [column][row] so that consecutive Δ3 read consecutive doubles.
-__global__ void ls_reduce_kernel(const LsReduceJob *__restrict__ jobs)
+// slots) of the partial tiles, TwoSum-compensated, in a fixed order: RED_PARTS threads a cell each add an
+// equal run of the terms, eight loads ahead of their sums, and the first adds the runs' sums in order.
+// Partial tiles are [column][row] so that consecutive Δ3 read consecutive doubles.  Bound by the latency of
+// a cell's chain of loads, not by bytes: 282 terms a cell (46 triangles of 32 channels, eight launches) took
+// 0.79 ms with one thread a cell.
+constexpr int RED_PARTS = 8;
+
+__global__ void __launch_bounds__(32 * RED_PARTS) ls_reduce_kernel(const LsReduceJob *__restrict__ jobs)
 {
+    __shared__ double ssum[RED_PARTS][32], scomp[RED_PARTS][32];
     const LsReduceJob j = jobs[blockIdx.y];
     const long ncsize = (long)j.nclen * j.nclen;
-    const long d = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (d >= ncsize) return;
-    const int d2 = (int)(d / j.nclen), d3 = (int)(d % j.nclen);
+    const int lane = threadIdx.x, part = threadIdx.y;
+    const long d = (long)blockIdx.x * 32 + lane;
     constexpr long TILE = (long)LS_ROWS * LS_ROWS;
     double s = 0.0, comp = 0.0;
     auto add = [&](double v) {
@@ -27,15 +32,46 @@ __global__ void ls_reduce_kernel(const LsReduceJob *__restrict__ jobs)
         comp += (s - (t - bp)) + (v - bp);
         s = t;
     };
-    if (j.k > 1) {
-        for (int u = 0; u < j.nab * j.V; ++u) {
-            const double *p = j.partial + u * TILE + (long)d2 * LS_ROWS;
-            for (int a = 0; a < j.k; ++a) add(p[a * j.rs + d3]);
+    if (d < ncsize) {
+        const int d2 = (int)(d / j.nclen), d3 = (int)(d % j.nclen);
+        const int n = j.nab * j.V * j.k;
+        const int i0 = (int)((long)n * part / RED_PARTS), i1 = (int)((long)n * (part + 1) / RED_PARTS);
+        // term i: unit i / k, slot i % k (k = 1 for a wide window's tile pair)
+        const double *p;
+        if (j.k > 1) {
+            p = j.partial + (long)d2 * LS_ROWS + d3;
+        } else {
+            const int t2 = d2 / LS_ROWS, t3 = d3 / LS_ROWS;
+            p = j.partial + (long)(t3 * j.T + t2) * j.nab * j.V * TILE + (long)(d2 % LS_ROWS) * LS_ROWS + d3 % LS_ROWS;
         }
-    } else {
-        const int t2 = d2 / LS_ROWS, c = d2 % LS_ROWS, t3 = d3 / LS_ROWS, r = d3 % LS_ROWS;
-        const long u0 = (long)(t3 * j.T + t2) * j.nab * j.V;
-        for (int u = 0; u < j.nab * j.V; ++u) add(j.partial[(u0 + u) * TILE + (long)c * LS_ROWS + r]);
+        p += (i0 / j.k) * TILE + (i0 % j.k) * j.rs;
+        int slot = i0 % j.k;
+        auto next = [&] {
+            const double v = *p;
+            p += j.rs;
+            if (++slot == j.k) {
+                slot = 0;
+                p += TILE - (long)j.k * j.rs;
+            }
+            return v;
+        };
+        int i = i0;
+        for (; i + 8 <= i1; i += 8) {
+            double v[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = next();
+#pragma unroll
+            for (int q = 0; q < 8; ++q) add(v[q]);
+        }
+        for (; i < i1; ++i) add(next());
+    }
+    ssum[part][lane] = s;
+    scomp[part][lane] = comp;
+    __syncthreads();
+    if (part != 0 || d >= ncsize) return;
+    for (int q = 1; q < RED_PARTS; ++q) {
+        add(ssum[q][lane]);
+        comp += scomp[q][lane];
     }
     j.lag[d] = s + comp;
 }
@@ -49,7 +85,7 @@ int LsShape::cols(int t2) const
 }
 int LsShape::lag_cols(int t2) const { return k > 1 ? nclen : std::min(LS_ROWS, nclen - LS_ROWS * t2); }
 
-LsShape ls_shape(int nc, int nc10, long k_px, int sms, long min_bpu, long force_bpu)
+LsShape ls_shape(int nc, int nc10, long k_px, int sms, long min_groups, long force_bpu)
 {
     LsShape s;
     s.nc = nc;
@@ -66,8 +102,12 @@ LsShape ls_shape(int nc, int nc10, long k_px, int sms, long min_bpu, long force_
     s.AB = std::max(1, std::min({nc, LS_SPAN - span_extra, LS_ROWS * s.k}));
     s.nab = (nc + s.AB - 1) / s.AB;
     s.nblk = std::max<long>(1, (k_px + LS_BLOCK - 1) / LS_BLOCK);
-    // Units: about six per SM for a large job, so the last wave is short; at least min_bpu blocks
-    // each (a unit's partial tile costs a write and a read of 128 KB).
+    // Units: about six per SM for a large job, so the last wave is short; each of at least min_groups
+    // anchor groups × blocks, so that a small job still spreads over the SMs: at eight blocks a unit, the
+    // kernel of one 2304-pixel triangle of 16 channels (9 blocks) took 104 µs on two SMs, and the eight
+    // launches of a 32-channel realisation's 46 triangles 4.0 ms against 2.4 ms at one block a unit.
+    const long per_block = std::max(1, s.AB / s.k) + 2;
+    const long min_bpu = std::max<long>(1, (min_groups + per_block - 1) / per_block);
     const long combos = (long)s.T * s.T * s.nab;
     const long target = 6L * std::max(1, sms);
     s.bpu = force_bpu > 0 ? std::min(s.nblk, force_bpu)
@@ -76,10 +116,10 @@ LsShape ls_shape(int nc, int nc10, long k_px, int sms, long min_bpu, long force_
     return s;
 }
 
-void ls_plan_job(LsJobPlan &p, int nc, int nc10, long k_px, const std::vector<int> &weight, int sms, long min_bpu,
+void ls_plan_job(LsJobPlan &p, int nc, int nc10, long k_px, const std::vector<int> &weight, int sms, long min_groups,
                  long force_bpu)
 {
-    p.s = ls_shape(nc, nc10, k_px, sms, min_bpu, force_bpu);
+    p.s = ls_shape(nc, nc10, k_px, sms, min_groups, force_bpu);
     p.groups.clear();
     p.group_off.assign(1, 0);
     for (int ab = 0; ab < p.s.nab; ++ab) {
@@ -128,7 +168,7 @@ int ls_reduce(amber_cuda_ctx *c, const std::vector<LsReduceJob> &jobs)
     phase_begin(c, 2);
     for (size_t j0 = 0; j0 < jobs.size(); j0 += 65535) {
         const unsigned nj = (unsigned)std::min<size_t>(65535, jobs.size() - j0);
-        ls_reduce_kernel<<<dim3((unsigned)((cells + 255) / 256), nj), 256, 0, c->stream>>>(
+        ls_reduce_kernel<<<dim3((unsigned)((cells + 31) / 32), nj), dim3(32, RED_PARTS), 0, c->stream>>>(
             (const LsReduceJob *)c->lsred.p + j0);
         c->launches += 1;
     }
