@@ -375,6 +375,10 @@ int run_next_batch(amber_cuda_ctx *c, RunState &st, std::vector<I8Job> *jobs)
             job.hi.push_back(c->uhigh[r]);
         }
         carve(pass == 0 ? c->maps_d.p : c->maps_i.p, job, &dmaps[pass]);
+        if (prec == AMBER_PREC_MIXED) {
+            job.need_dig.assign(ms.nslots, 0);
+            for (int t : batch) job.need_dig[ms.slot_of_ring[tri[3 * t + 1]]] = 1;
+        }
         phase_begin(c, 0);
         rc = build_maps(c, job);
         phase_end(c);

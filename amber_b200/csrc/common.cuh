@@ -140,6 +140,7 @@ struct MapJob {
     const int *weight;            // device multiplicities of the source channels (mixed path)
     int8_t *dig;                  // mixed path: digit planes [slot][3][kp/16][nch][16] (kp multiple of 256)
     int *bexp;                    // mixed path: exponent per (slot, 256-pixel block)
+    std::vector<char> need_dig;   // mixed path: slots whose digit planes are read (empty: all)
 };
 int build_maps(amber_cuda_ctx *c, const MapJob &job);
 

@@ -177,94 +177,160 @@ __device__ __forceinline__ uint16_t bf16_bits(float f)
     return *reinterpret_cast<uint16_t *>(&b);
 }
 
-template <int C>
-__global__ void __launch_bounds__(kThreads) ring_rows_kernel(const double2 *__restrict__ Y, long ng, int jmax,
-                                                              const RingMeta meta, long nch,
-                                                              const double2 *__restrict__ tw_g, long kp,
-                                                              double *__restrict__ out_f64,
-                                                              uint16_t *__restrict__ out_hi,
-                                                              uint16_t *__restrict__ out_lo,
-                                                              float *__restrict__ out_f32,
-                                                              const int *__restrict__ weight)
+// D(16×8) += A(16×8) · B(8×8), FP64.  Fragments (g = lane / 4, t = lane % 4): A {(g, t), (g+8, t),
+// (g, t+4), (g+8, t+4)}, B {(t, g), (t+4, g)}, C {(g, 2t), (g, 2t+1), (g+8, 2t), (g+8, 2t+1)}.
+__device__ __forceinline__ void dmma(double (&c)[4], const double (&a)[4], double b0, double b1)
+{
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                 "{%0, %1, %2, %3};"
+                 : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+                 : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
+}
+
+// Pass 2 as an FP64 GEMM over (pixel x ≤ Ng/4) × (column = output row n0, channel) with j as the
+// contraction: with C_e, C_o the sums of Re Y·cos over even and odd j and S_e, S_o those of Im Y·sin, one
+// quarter of the row gives the whole row (h = Ng/2; Ng is even):
+//     D[x] = C_e + C_o − S_e − S_o,   D[Ng − x] = C_e + C_o + S_e + S_o,
+//     D[h − x] = C_e − C_o + S_e − S_o,   D[h + x] = C_e − C_o − S_e + S_o,
+// i.e. half an FMA per pixel and j.  A CTA holds RC columns' spectrum rows in shared memory; two warps share
+// every fourth tile of 16 x, half the columns each.  The A fragments (cos, sin of j·x) come from the twiddle table, at indices that
+// advance by 16·x mod Ng per step of 16 j, and serve RN column tiles.  Bound by the FP64 pipe for wide
+// rings and by the map stores for narrow ones.  On the FP64 cores with two FMAs per pixel and j, each fed by a
+// shared load of its own, fourteen rings of 128 channels on 740 × 740 pixels took 13.6 ms; now 3.0 ms.
+constexpr int RC = 32;       // columns per CTA
+constexpr int RS = RC + 1;   // their stride in shared memory: odd, so that a fragment load is conflict-free
+constexpr int RN = RC / 16;  // column tiles (of 8) per warp
+constexpr int RROWS_THREADS = 256;
+constexpr int RX = 16 * (RROWS_THREADS / 64);  // x per round of the CTA's warps
+
+__global__ void __launch_bounds__(RROWS_THREADS, 2) ring_rows_kernel(const double2 *__restrict__ Y, int ng, int jmax,
+                                                                      const RingMeta meta, long nch,
+                                                                      const double2 *__restrict__ tw_g, long kp, int jstage,
+                                                                      double *__restrict__ out_f64,
+                                                                      uint16_t *__restrict__ out_hi,
+                                                                      uint16_t *__restrict__ out_lo,
+                                                                      float *__restrict__ out_f32,
+                                                                      const int *__restrict__ weight)
 {
     extern __shared__ double2 smem[];
     double2 *tw = smem;       // ng
-    double2 *ys = tw + ng;    // J × C
-    const long n0 = blockIdx.x;
+    double2 *ys = tw + ng;    // [jstage][RS]: all of the ring's J, or a run of them at a time
     const int s = blockIdx.y;
-    const long q0 = (long)blockIdx.z * C;
-    const int J = meta.jc[s];
+    const long col0 = (long)blockIdx.x * RC, ncol = (long)ng * nch;
+    const int J = meta.jc[s], steps = (J + 15) / 16;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (long i = tid; i < ng; i += kThreads) tw[i] = tw_g[i];
-    for (int e = tid; e < J * C; e += kThreads) {
-        int jj = e / C, q = e % C;
-        double2 v = make_double2(0.0, 0.0);
-        if (q0 + q < nch) v = Y[(((long)s * ng + n0) * jmax + jj) * nch + q0 + q];
-        if (jj == 0) v.y = 0.0;  // c2r ignores Im of the DC bin
-        else { v.x *= 2.0; v.y *= 2.0; }
-        ys[e] = v;
-    }
+    for (int i = tid; i < ng; i += RROWS_THREADS) tw[i] = tw_g[i];
+    // this thread's column of the staged spectrum (RROWS_THREADS is a multiple of RC)
+    const int sc = tid % RC;
+    const long scol = col0 + sc;
+    const double2 *src = Y + (((long)s * ng + scol / nch) * jmax) * nch + scol % nch;
+    auto stage = [&](int j0) {
+        const int n = min(jstage, 16 * steps - j0);
+        for (int j = tid / RC; j < n; j += RROWS_THREADS / RC) {
+            double2 v = make_double2(0.0, 0.0);
+            if (j0 + j < J && scol < ncol) v = src[(long)(j0 + j) * nch];
+            if (j0 + j == 0) v.y = 0.0;  // c2r ignores Im of the DC bin
+            else { v.x *= 2.0; v.y *= 2.0; }
+            ys[j * RS + sc] = v;
+        }
+    };
+    stage(0);
     __syncthreads();
 
-    constexpr int G = 32 / C;
-    // A thread evaluates R pixel pairs (x, Ng − x): they share each twiddle, cos and −sin,
-    // so one shared-memory load and one index step feed four FMAs.  x runs over [0, Ng/2];
-    // for x = 0 and x = Ng/2 the pair is one pixel.
-    constexpr int R = 4;
-    const int q = lane % C, g = lane / C;
-    const int gid = warp * G + g;
-    const int ngroups = (kThreads / 32) * G;
-    const long npair = ng / 2 + 1;
-    const long slot_row = ((long)s * nch + q0 + q) * kp + n0 * ng;
-    // the mixed path's fp32 maps carry the channel multiplicity (0 for flagged channels)
-    const double wq = (weight && q0 + q < nch) ? (double)weight[q0 + q] : 1.0;
-    for (long nb = gid; nb * R < npair; nb += ngroups) {
-        double acc[R], accm[R];  // pixel x, pixel Ng − x
-        int idx[R], step[R];
+    const int g = lane >> 2, t = lane & 3;
+    const int h = ng / 2, xmax = h / 2, nb = (warp & 1) * 8 * RN;  // first column of this warp
+    // the columns this thread stores: row origin (−1: past the last column) and channel multiplicity (the
+    // mixed path's fp32 maps carry it, 0 for flagged channels)
+    long at[2 * RN];
+    double wq[2 * RN];
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            long x = nb * R + r;
-            step[r] = (int)(x < npair ? x : 0);
-            idx[r] = 0;
-            acc[r] = 0.0;
-            accm[r] = 0.0;
+    for (int i = 0; i < 2 * RN; ++i) {
+        const unsigned col = (unsigned)(col0 + nb + 8 * (i / 2) + 2 * t + i % 2);
+        const unsigned n0 = col / (unsigned)nch, ch = col % (unsigned)nch;
+        at[i] = col < (unsigned)ncol ? ((long)s * nch + ch) * kp + (long)n0 * ng : -1;
+        wq[i] = weight && col < (unsigned)ncol ? (double)weight[ch] : 1.0;
+    }
+    for (int xg = 0; xg <= xmax; xg += RX) {
+        const int x0 = xg + 16 * (warp >> 1);
+        // twiddle indices of j = 2t and 2t + 8 for the lane's two x (clamped: rows past xmax are not stored)
+        const int xa[2] = {min(x0 + g, xmax), min(x0 + g + 8, xmax)};
+        int idx[2][2], d16[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            idx[i][0] = (2 * t * xa[i]) % ng;
+            idx[i][1] = ((2 * t + 8) * xa[i]) % ng;
+            d16[i] = (16 * xa[i]) % ng;
         }
-        for (int jj = 0; jj < J; ++jj) {
-            double2 y = ys[jj * C + q];
+        double ce[RN][4], co[RN][4], se[RN][4], so[RN][4];
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                double2 w = tw[idx[r]];
-                acc[r] = fma(y.x, w.x, acc[r]);
-                acc[r] = fma(-y.y, w.y, acc[r]);
-                accm[r] = fma(y.x, w.x, accm[r]);
-                accm[r] = fma(y.y, w.y, accm[r]);
-                int t = idx[r] + step[r];
-                idx[r] = t >= ng ? t - (int)ng : t;
+        for (int n = 0; n < RN; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) ce[n][e] = co[n][e] = se[n][e] = so[n][e] = 0.0;
+        const double2 *yj = ys + 2 * t * RS + nb + g;
+        for (int st = 0, left = jstage / 16; st < steps; ++st, yj += 16 * RS) {
+            if (left-- == 0) {  // a ring too wide for one stage: its next run of j
+                __syncthreads();
+                stage(16 * st);
+                __syncthreads();
+                left = jstage / 16 - 1;
+                yj = ys + 2 * t * RS + nb + g;
+            }
+            double ac[4], as[4], bc[4], bs[4];  // cos, sin at even and at odd j
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const double2 w = tw[idx[i][kk]];
+                    int o = idx[i][kk] + xa[i];
+                    o = o >= ng ? o - ng : o;
+                    const double2 v = tw[o];
+                    ac[2 * kk + i] = w.x;
+                    as[2 * kk + i] = w.y;
+                    bc[2 * kk + i] = v.x;
+                    bs[2 * kk + i] = v.y;
+                    o = idx[i][kk] + d16[i];
+                    idx[i][kk] = o >= ng ? o - ng : o;
+                }
+#pragma unroll
+            for (int n = 0; n < RN; ++n) {
+                const double2 e0 = yj[8 * n], e1 = yj[8 * RS + 8 * n];
+                const double2 o0 = yj[RS + 8 * n], o1 = yj[9 * RS + 8 * n];
+                dmma(ce[n], ac, e0.x, e1.x);
+                dmma(se[n], as, e0.y, e1.y);
+                dmma(co[n], bc, o0.x, o1.x);
+                dmma(so[n], bs, o0.y, o1.y);
             }
         }
-        if (q0 + q < nch) {
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const long x = nb * R + r;
-                if (x >= npair) continue;
+        for (int n = 0; n < RN; ++n)
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const long n1 = h == 0 ? x : ng - x;
-                    if (h == 1 && (x == 0 || n1 == x)) continue;
-                    const long o = slot_row + n1;
-                    const double v = h == 0 ? acc[r] : accm[r];
-                    if (out_f64) out_f64[o] = v;
-                    if (out_f32) out_f32[o] = (float)(v * wq);
+            for (int e = 0; e < 4; ++e) {
+                const int x = x0 + g + 8 * (e >> 1), i = 2 * n + (e & 1);
+                const long o = at[i];
+                if (x > xmax || o < 0) continue;
+                const double cp = ce[n][e] + co[n][e], cm = ce[n][e] - co[n][e];
+                const double sp = se[n][e] + so[n][e], sm = se[n][e] - so[n][e];
+                auto put = [&](int n1, double v) {
+                    if (out_f64) out_f64[o + n1] = v;
+                    if (out_f32) out_f32[o + n1] = (float)(v * wq[i]);
                     if (out_hi) {
                         // split: hi = bf16(v), lo = bf16(v − hi) (both round-to-nearest)
-                        float f = (float)v;
-                        uint16_t hb = bf16_bits(f);
-                        float hf = __uint_as_float((uint32_t)hb << 16);
-                        out_hi[o] = hb;
-                        out_lo[o] = bf16_bits((float)(v - (double)hf));
+                        const uint16_t hb = bf16_bits((float)v);
+                        out_hi[o + n1] = hb;
+                        out_lo[o + n1] = bf16_bits((float)(v - (double)__uint_as_float((uint32_t)hb << 16)));
                     }
+                };
+                put(x, cp - sp);
+                if (x > 0) put(ng - x, cp + sp);
+                if (2 * x < h) {
+                    put(h - x, cm + sm);
+                    if (x > 0) put(h + x, cm - sm);
                 }
             }
+        if (16 * steps > jstage && xg + RX <= xmax) {
+            __syncthreads();
+            stage(0);
+            __syncthreads();
         }
     }
 }
@@ -315,28 +381,38 @@ __global__ void __launch_bounds__(LS_BLOCK) block_expo_kernel(const float *__res
     }
 }
 
-// Three digit planes per slot in the contraction's staging order,
+// Slots of one quantize launch: the rings that stand second in a triangle of the batch (the contraction reads
+// no other ring's digits), which of the rings of a batch is often a quarter.
+struct SlotList {
+    unsigned char s[256];
+};
+
+// Three digit planes per listed slot in the contraction's staging order,
 // dig[s][digit][x/16][ch][16 pixels]: a TMA box of consecutive channels and two 16-pixel
 // groups then lands in shared memory exactly as the MMA reads a K-major operand without
 // swizzle (8-row core matrices of 16 bytes).  Pixels at or past k become zero digits.
 __global__ void __launch_bounds__(256) quantize_kernel(const float *__restrict__ f32, const int *__restrict__ bexp,
                                                        long k, long kp, long nch, long nblk,
-                                                       int8_t *__restrict__ dig)
+                                                       const SlotList slots, int8_t *__restrict__ dig)
 {
     const long b = blockIdx.x;
-    const int s = blockIdx.y;
+    const int s = slots.s[blockIdx.y];
     const float sc = ldexpf(127.f, -bexp[(long)s * nblk + b]);
     const long kpg = kp / 16;
     for (long e = threadIdx.x; e < (LS_BLOCK / 16) * nch; e += blockDim.x) {
         const long g = e / nch, ch = e % nch;
         const long x0 = b * LS_BLOCK + g * 16;
-        const float *src = f32 + ((long)s * nch + ch) * kp + x0;
+        const float4 *src = reinterpret_cast<const float4 *>(f32 + ((long)s * nch + ch) * kp + x0);
         uint32_t w[3][4];
+        float4 in[4];  // rows are kp ≡ 0 (mod 256) floats from a 256-byte boundary: 16-byte loads, and past k too
+#pragma unroll
+        for (int q = 0; q < 4; ++q) in[q] = src[q];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
+            const float v[4] = {in[q].x, in[q].y, in[q].z, in[q].w};
             uint32_t a[4], bb[4], cc[4];
 #pragma unroll
-            for (int t = 0; t < 4; ++t) digits254(x0 + 4 * q + t < k ? src[4 * q + t] * sc : 0.f, a[t], bb[t], cc[t]);
+            for (int t = 0; t < 4; ++t) digits254(x0 + 4 * q + t < k ? v[t] * sc : 0.f, a[t], bb[t], cc[t]);
             w[0][q] = __byte_perm(__byte_perm(a[0], a[1], 0x0040), __byte_perm(a[2], a[3], 0x0040), 0x5410);
             w[1][q] = __byte_perm(__byte_perm(bb[0], bb[1], 0x0040), __byte_perm(bb[2], bb[3], 0x0040), 0x5410);
             w[2][q] = __byte_perm(__byte_perm(cc[0], cc[1], 0x0040), __byte_perm(cc[2], cc[3], 0x0040), 0x5410);
@@ -395,10 +471,10 @@ int build_maps(amber_cuda_ctx *c, const MapJob &job)
     while (C1 > 1 && p1_smem(C1) > smem_cap) C1 /= 2;
     if (p1_smem(C1) > smem_cap) return fail(c, AMBER_ERR_ARG, "ring too wide for the column stage (%d rows)", rows_max);
     const size_t s1 = p1_smem(C1);
-    auto p2_smem = [&](int C) { return sizeof(double2) * ng + sizeof(double2) * C * jmax; };
-    int C2 = 32;
-    while (C2 > 1 && p2_smem(C2) > smem_cap) C2 /= 2;
-    const size_t s2 = p2_smem(C2);
+    // pass 2: a stage of j that leaves room for two CTAs an SM where the widest ring fits it
+    const size_t s2_cap = std::max((size_t)112 * 1024, sizeof(double2) * ((size_t)ng + 16 * RS));
+    const int jstage = (int)std::min<size_t>((jmax + 15) / 16, (s2_cap / sizeof(double2) - ng) / (16 * RS)) * 16;
+    const size_t s2 = sizeof(double2) * ((size_t)ng + (size_t)jstage * RS);
     // up to RING_META_MAX slots per launch pair, each launch's pointers offset to its first slot
     for (int sb = 0; sb < job.nslots; sb += RING_META_MAX) {
         const int ns = std::min(RING_META_MAX, job.nslots - sb);
@@ -433,22 +509,9 @@ int build_maps(amber_cuda_ctx *c, const MapJob &job)
         c->launches += 1;
         if ((rc = cuda_check(c, cudaGetLastError(), "ring_cols_kernel launch"))) return rc;
 
-        dim3 g2((unsigned)ng, ns, (unsigned)((job.nch + C2 - 1) / C2));
-#define LAUNCH_ROWS(CC)                                                                                        \
-    do {                                                                                                        \
-        cudaFuncSetAttribute(ring_rows_kernel<CC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2);        \
-        ring_rows_kernel<CC><<<g2, kThreads, s2, c->stream>>>(Ys, ng, jmax, meta, job.nch, tw, job.kp, of64, ohi, \
-                                                               olo, of32, job.weight);                           \
-    } while (0)
-        switch (C2) {
-            case 32: LAUNCH_ROWS(32); break;
-            case 16: LAUNCH_ROWS(16); break;
-            case 8: LAUNCH_ROWS(8); break;
-            case 4: LAUNCH_ROWS(4); break;
-            case 2: LAUNCH_ROWS(2); break;
-            default: LAUNCH_ROWS(1); break;
-        }
-#undef LAUNCH_ROWS
+        cudaFuncSetAttribute(ring_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2);
+        ring_rows_kernel<<<dim3((unsigned)((ng * job.nch + RC - 1) / RC), ns), RROWS_THREADS, s2, c->stream>>>(
+            Ys, (int)ng, jmax, meta, job.nch, tw, job.kp, jstage, of64, ohi, olo, of32, job.weight);
         c->launches += 1;
         if ((rc = cuda_check(c, cudaGetLastError(), "ring_rows_kernel launch"))) return rc;
     }
@@ -456,8 +519,14 @@ int build_maps(amber_cuda_ctx *c, const MapJob &job)
         const long nblk = job.kp / LS_BLOCK;
         dim3 gq((unsigned)nblk, (unsigned)job.nslots);
         block_expo_kernel<<<gq, LS_BLOCK, 0, c->stream>>>(job.out_f32, ng * ng, job.kp, job.nch, nblk, job.bexp);
-        quantize_kernel<<<gq, 256, 0, c->stream>>>(job.out_f32, job.bexp, ng * ng, job.kp, job.nch, nblk, job.dig);
-        c->launches += 2;
+        SlotList list;
+        unsigned n = 0;
+        for (int s = 0; s < job.nslots; ++s)
+            if (job.need_dig.empty() || job.need_dig[s]) list.s[n++] = (unsigned char)s;
+        if (n > 0)
+            quantize_kernel<<<dim3((unsigned)nblk, n), 256, 0, c->stream>>>(job.out_f32, job.bexp, ng * ng, job.kp,
+                                                                            job.nch, nblk, list, job.dig);
+        c->launches += n > 0 ? 2 : 1;
         rc = cuda_check(c, cudaGetLastError(), "quantize_kernel launch");
     }
     return rc;
