@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(F_NT, 1) ls_fp64_kernel(const F64Desc *__restr
         }
     }
     // the unit's partial tile [column][row]; slot a of a packed tile lands at lag column c − a
-    double *out = partial + u.tile * (long)(LS_ROWS * LS_ROWS);
+    double *out = partial + u.tile;
     const int lagc = ks > 1 ? nclen : ncols;
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt)
@@ -328,29 +328,28 @@ int contract_fp64_jobs(amber_cuda_ctx *c, const std::vector<F64Job> &jobs)
                 return rc;
         return AMBER_OK;
     }
-    constexpr size_t TILE_B = sizeof(double) * LS_ROWS * LS_ROWS;
     // partial tiles of one launch: no more than the context's budget leaves beside its maps (less a margin
     // for the job lists); a job too large for that on its own takes longer runs of blocks per unit
     const size_t room = (c->budget > c->held ? c->budget - c->held : 0) + c->partial.bytes, margin = (size_t)8 << 20;
     const size_t pcap = std::min(std::max<size_t>((size_t)256 << 20, contract_partial_cap(c)),
                                  room > margin ? room - margin : 0);
-    const long tile_cap = std::max<long>(1, (long)(pcap / TILE_B));
+    const long cap = (long)(pcap / sizeof(double));
     size_t j0 = 0;
     while (j0 < jobs.size()) {
         // plan as many jobs as their partial tiles allow in one launch
         std::vector<LsJobPlan> plans;
-        long tiles = 0;
+        long used = 0;  // doubles of partial tiles
         size_t j1 = j0;
         for (; j1 < jobs.size(); ++j1) {
             LsJobPlan p;
             ls_plan_job(p, (int)c->nc, c->nc10, jobs[j1].k, c->weight, c->num_sms, 1, ls_force_bpu(c->chunk_px));
-            if (j1 > j0 && tiles + p.s.units() > tile_cap) break;
-            if (p.s.units() > tile_cap && c->chunk_px <= 0) {
-                const long runs = std::max<long>(1, tile_cap / (p.s.units() / p.s.V));
+            if (j1 > j0 && used + p.s.units() * p.s.tile() > cap) break;
+            if (p.s.units() * p.s.tile() > cap && c->chunk_px <= 0) {
+                const long runs = std::max<long>(1, cap / p.s.tile() / (p.s.units() / p.s.V));
                 ls_plan_job(p, (int)c->nc, c->nc10, jobs[j1].k, c->weight, c->num_sms, 1, (p.s.nblk + runs - 1) / runs);
             }
-            p.unit_base = tiles;
-            tiles += p.s.units();
+            p.unit_base = used;
+            used += p.s.units() * p.s.tile();
             plans.push_back(std::move(p));
         }
         std::vector<LsUnit> units;
@@ -367,7 +366,7 @@ int contract_fp64_jobs(amber_cuda_ctx *c, const std::vector<F64Job> &jobs)
         const size_t off_u = (desc_b + 255) / 256 * 256, off_g = off_u + (unit_b + 255) / 256 * 256;
         const size_t off_o = off_g + (sizeof(int) * ngroups + 255) / 256 * 256;
         const size_t stage_b = off_o + sizeof(int) * noff;
-        if ((rc = ensure(c, c->partial, (size_t)tiles * TILE_B, "partial lag tiles"))) return rc;
+        if ((rc = ensure(c, c->partial, sizeof(double) * (size_t)used, "partial lag tiles"))) return rc;
         if ((rc = ensure(c, c->jobdesc, stage_b, "job list"))) return rc;
         if ((rc = cuda_check(c, cudaStreamSynchronize(c->stream), "job staging"))) return rc;
         if (c->stage_bytes < stage_b) {
@@ -396,8 +395,8 @@ int contract_fp64_jobs(amber_cuda_ctx *c, const std::vector<F64Job> &jobs)
             for (size_t q = 0; q < p.group_off.size(); ++q) ho[opos + q] = p.group_off[q];
             gpos += p.groups.size();
             opos += p.group_off.size();
-            red.push_back(LsReduceJob{(const double *)c->partial.p + p.unit_base * LS_ROWS * LS_ROWS, jb.lag_out, nclen,
-                                      p.s.k, p.s.rs, p.s.T, p.s.nab, p.s.V});
+            red.push_back(LsReduceJob{(const double *)c->partial.p + p.unit_base, jb.lag_out, nclen,
+                                      p.s.k, p.s.rs, p.s.T, p.s.nab, p.s.V, p.s.tile()});
         }
         std::copy(units.begin(), units.end(), (LsUnit *)(h + off_u));
         if ((rc = cuda_check(c, cudaMemcpyAsync(d, h, stage_b, cudaMemcpyHostToDevice, c->stream), "job list upload")))

@@ -18,9 +18,9 @@
 //     Σ_x (w1D1)(w2D2)(w3D3) = 2^(E1+E2+E3)/127² · Σ_k 254^−k Σ_{i+j=k} Σ_x Q_i P_j.
 // Class k accumulates in its own int32 TMEM accumulator.  Classes 0-2 (six
 // MMAs per 32 pixels) bound the D-map error near 1e-7 of Σ|products|; the
-// peaked sampling-mask maps also need class 3 (P3·Q0 + P2·Q1 + P1·Q2): the
-// three accumulators of classes 0-2 at N = 128 plus the A staging fill TMEM,
-// so a mask block runs a second sweep that forms digits 1-3 of the product
+// peaked sampling-mask maps also need class 3 (P3·Q0 + P2·Q1 + P1·Q2).  Up to
+// N = 96 four accumulators and four-digit A buffers fit TMEM, and a mask block runs
+// one sweep; at N = 128 it runs a second sweep that forms digits 1-3 of the product
 // and accumulates class 3 alone.  The numbers behind this choice: a numpy
 // emulation of these exact digit operations on the single-realisation
 // workload's Ng1 = 354 and 740 maps gave 6–9e-8 (D, classes 0-2) and
@@ -90,11 +90,13 @@ constexpr int NMMA = 2;                      // MMA issuing warps
 constexpr int NTHREADS = (NFORM + 4) * 32;
 constexpr int TMEM_COLS = 512;
 constexpr int NSET = NFORM / 4;              // former sets: each anchor group is formed by one set of 4 warps
-constexpr int ABUF_COLS = 24;                // 3 digits × 8 columns (32 int8 per row per digit)
+constexpr int ABUF_COLS = 24;                // A buffer: 3 digits × 8 columns (32 int8 per row per digit)
+constexpr int ABUF4_COLS = 32;               // with four digits
 constexpr int NABUF_MAX = 8;                 // A buffers: as many as TMEM holds beside the accumulators
 constexpr long MIN_GROUPS = 5;                // least work of a unit (lagspace.cuh): ~10 µs
 constexpr int NSTAGE_MAX = 8;                // stages: as many as shared memory holds
 static_assert(3 * LS_ROWS + 5 * ABUF_COLS <= TMEM_COLS, "TMEM: five A buffers beside the widest accumulators");
+static_assert(NSET <= 4, "a set may be one use of a buffer ahead of the tensor pipe, not two: sets ≤ buffers");
 
 // Shared memory: barriers, hand-off counts and the unit's anchor groups, then the stages.
 constexpr int SM_FLAGS = 512;                // [NABUF_MAX] hand-off counts of the A buffers
@@ -113,7 +115,7 @@ struct alignas(64) I8Desc {
     long k;
     int nc, nc10, nclen, ks, rs, AB, T;
     int span3, span2;
-    int sweeps;                     // 1: classes 0-2; 2: also class 3 (mask maps)
+    int mask;                       // sampling-mask maps: class 3 as well
     uint32_t tx_bytes;              // bytes one slice's three TMA boxes deliver
     int nst, st_bytes, st_d1, st_d2;  // stages, bytes of one, offsets of its D1 rows and D2 digits (D3 first)
 };
@@ -263,10 +265,14 @@ struct IssueState {
 };
 
 // Issues the MMAs of one item (a pixel block, one sweep): every slice's anchor groups in order.
-// SECOND: which of the two issuing threads; class k = Σ_{i+j=k} Q_i·P_j.  SWEEP 0: classes 0 and 1 (first
-// thread) or 2 (second), the A buffer holds P0, P1, P2.  SWEEP 1: class 3 = P3·Q0 + P2·Q1 (first) + P1·Q2
-// (second), the A buffer holds P1, P2, P3.  The loop is kept to few instructions beside the MMAs: they
-// wait for issue slots behind the formers of the same SM partition.
+// SECOND: which of the two issuing threads; class k = Σ_{i+j=k} Q_i·P_j.
+//   SW_D: the A buffer holds P0, P1, P2; the first thread runs classes 0 and 1, the second class 2.
+//   SW_CLASS3: P1, P2, P3; class 3 = P3·Q0 + P2·Q1 (first) + P1·Q2 (second, an accumulator of its own).
+//   SW_MASK4: P0 .. P3; the first thread runs classes 0 and 3, the second classes 1 and 2.
+// The loop is kept to few instructions beside the MMAs: they wait for issue slots behind the formers of
+// the same SM partition.
+enum { SW_D, SW_CLASS3, SW_MASK4 };
+
 template <bool SECOND, int SWEEP>
 __device__ __forceinline__ bool issue_item(IssueState &t, int nsl, uint64_t *st_full, uint64_t *st_empty,
                                            volatile int *abort_flag, int *err)
@@ -279,8 +285,8 @@ __device__ __forceinline__ bool issue_item(IssueState &t, int nsl, uint64_t *st_
         uint4 e = lds_u128(first ? t.groups + 16 * t.ngr : t.groups);
         uint32_t next = t.groups;
         for (uint32_t g = 0; g < t.ngr; ++g) {
-            const uint32_t q0 = sd + e.x, q1 = q0 + t.ddig, q2 = q1 + t.ddig;
-            const uint32_t d = t.acc + e.y, idesc = e.z, a = t.a_first + t.ab * ABUF_COLS;
+            const uint32_t q0 = sd + e.x, q1 = q0 + t.ddig, q2 = q1 + t.ddig, qh = t.desc_hi;
+            const uint32_t d = t.acc + e.y, idesc = e.z, a = t.a_first + t.ab * (SWEEP == SW_MASK4 ? ABUF4_COLS : ABUF_COLS);
             const uint32_t bar = t.bars + t.ab * 8;
             next += 16;
             e = lds_u128(next);
@@ -288,28 +294,44 @@ __device__ __forceinline__ bool issue_item(IssueState &t, int nsl, uint64_t *st_
             fence_after();
             if (++t.ab == t.nabuf) { t.ab = 0; t.need += 4; }
             t.seen = count_load(t.flags + t.ab * 4);
-            if (first) {
-                if constexpr (SWEEP == 0 && !SECOND) {
-                    umma_i8<0>(d, a, q0, t.desc_hi, idesc);
-                    umma_i8<0>(d + t.nmma, a + 8, q0, t.desc_hi, idesc);
+            // the MMAs that may be the first into their accumulator, then the rest
+            auto leading = [&](auto addc) {
+                constexpr int ADD = decltype(addc)::value;
+                if constexpr (SWEEP == SW_D && !SECOND) {
+                    umma_i8<ADD>(d, a, q0, qh, idesc);
+                    umma_i8<ADD>(d + t.nmma, a + 8, q0, qh, idesc);
+                } else if constexpr (SWEEP == SW_D) {
+                    umma_i8<ADD>(d, a + 16, q0, qh, idesc);
+                } else if constexpr (SWEEP == SW_CLASS3 && !SECOND) {
+                    umma_i8<ADD>(d, a + 16, q0, qh, idesc);
+                } else if constexpr (SWEEP == SW_CLASS3) {
+                    umma_i8<ADD>(d, a, q2, qh, idesc);
+                } else if constexpr (!SECOND) {
+                    umma_i8<ADD>(d, a, q0, qh, idesc);
+                    umma_i8<ADD>(d + 3 * t.nmma, a + 24, q0, qh, idesc);
                 } else {
-                    umma_i8<0>(d, SECOND && SWEEP ? a : a + 16, SECOND && SWEEP ? q2 : q0, t.desc_hi, idesc);
+                    umma_i8<ADD>(d, a + 8, q0, qh, idesc);
+                    umma_i8<ADD>(d + t.nmma, a + 16, q0, qh, idesc);
                 }
-                first = false;
-            } else {
-                if constexpr (SWEEP == 0 && !SECOND) {
-                    umma_i8<1>(d, a, q0, t.desc_hi, idesc);
-                    umma_i8<1>(d + t.nmma, a + 8, q0, t.desc_hi, idesc);
-                } else {
-                    umma_i8<1>(d, SECOND && SWEEP ? a : a + 16, SECOND && SWEEP ? q2 : q0, t.desc_hi, idesc);
-                }
+            };
+            if (first) leading(std::integral_constant<int, 0>());
+            else leading(std::integral_constant<int, 1>());
+            first = false;
+            if constexpr (SWEEP == SW_D && !SECOND) {
+                umma_i8<1>(d + t.nmma, a, q1, qh, idesc);
+            } else if constexpr (SWEEP == SW_D) {
+                umma_i8<1>(d, a + 8, q1, qh, idesc);
+                umma_i8<1>(d, a, q2, qh, idesc);
+            } else if constexpr (SWEEP == SW_CLASS3 && !SECOND) {
+                umma_i8<1>(d, a + 8, q1, qh, idesc);
+            } else if constexpr (SWEEP == SW_MASK4 && !SECOND) {
+                umma_i8<1>(d + 3 * t.nmma, a + 16, q1, qh, idesc);
+                umma_i8<1>(d + 3 * t.nmma, a + 8, q2, qh, idesc);
+            } else if constexpr (SWEEP == SW_MASK4) {
+                umma_i8<1>(d, a, q1, qh, idesc);
+                umma_i8<1>(d + t.nmma, a + 8, q1, qh, idesc);
+                umma_i8<1>(d + t.nmma, a, q2, qh, idesc);
             }
-            if constexpr (SWEEP == 0 && !SECOND) umma_i8<1>(d + t.nmma, a, q1, t.desc_hi, idesc);
-            if constexpr (SWEEP == 0 && SECOND) {
-                umma_i8<1>(d, a + 8, q1, t.desc_hi, idesc);
-                umma_i8<1>(d, a, q2, t.desc_hi, idesc);
-            }
-            if constexpr (SWEEP == 1 && !SECOND) umma_i8<1>(d, a + 8, q1, t.desc_hi, idesc);
             umma_commit_bar(bar);
         }
         umma_commit_bar(smem_u32(&st_empty[t.s]));
@@ -318,6 +340,12 @@ __device__ __forceinline__ bool issue_item(IssueState &t, int nsl, uint64_t *st_
     return true;
 }
 
+// Whether a mask job's four class accumulators and four four-digit A buffers fit TMEM at MMA width nmma (≤ 96).
+__host__ __device__ constexpr bool mask4_fits(int nmma) { return 4 * nmma + NSET * ABUF4_COLS <= TMEM_COLS; }
+
+// FOUR: the launch's jobs are mask jobs run in one SW_MASK4 sweep (a kernel of its own: sharing one with the
+// three-digit sweeps cost those 9 % in register spills).
+template <bool FOUR>
 __global__ void __launch_bounds__(NTHREADS, 1)
     ls_i8_kernel(const I8Desc *__restrict__ jobs, const LsUnit *__restrict__ units, double *__restrict__ partial,
                  int *err)
@@ -345,9 +373,15 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     const int ncols = ks > 1 ? nclen : min(LS_ROWS, nclen - toff2);  // lag columns
     const int nwin = ks > 1 ? nclen + ks - 1 : ncols;                // window rows of D2
     const int nmma = ((nwin + 15) / 16) * 16;                        // MMA N
-    const int nabuf = min(NABUF_MAX, (TMEM_COLS - 3 * nmma) / ABUF_COLS);
+    // Sweeps of an item: classes 0-2 alone (SW_D); for the mask maps all four classes at once where four
+    // accumulators and four four-digit buffers fit TMEM (SW_MASK4: N ≤ 96), else classes 0-2 and then class 3
+    // from digits formed again (SW_D, SW_CLASS3).  One sweep with four digits takes 1.25 times a sweep with three
+    // where two took 2.2 times (realisations of 24-97 channels).
+    const int sweeps = jd->mask && !FOUR ? 2 : 1;
+    constexpr int abuf_cols = FOUR ? ABUF4_COLS : ABUF_COLS, ncls = FOUR ? 4 : 3;
+    const int nabuf = min(NABUF_MAX, (TMEM_COLS - ncls * nmma) / abuf_cols);
     const int nst = jd->nst, st_bytes = jd->st_bytes;
-    double *out = partial + u.tile * (long)(LS_ROWS * LS_ROWS);
+    double *out = partial + u.tile;
 
     // The unit's anchor groups {D2 descriptor offset, accumulator column, MMA instruction descriptor,
     // 16 × staged row of the first channel and mask of live 8-row blocks}.  Columns whose D2 channel lies outside [0, nc) add nothing, so a group's
@@ -410,10 +444,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t a_col0 = tmem + 3 * nmma;
+    const uint32_t a_col0 = tmem + ncls * nmma;
     const int ngr = *ngroups_s;
     bool ok = true;
-    const int sweeps = jd->sweeps;
     const long k = jd->k;
     auto nslices = [&](long b) {
         const long n = (k - b * LS_BLOCK + SLICE - 1) / SLICE;
@@ -422,7 +455,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 
     if (ngr == 0) {
         // no anchor of the block has a channel in range: the partial tile is zero
-        for (int e = tid; e < LS_ROWS * LS_ROWS; e += NTHREADS) out[e] = 0.0;
+        for (int e = tid; e < LS_ROWS * ncols; e += NTHREADS) out[e] = 0.0;
     } else if (warp == WARP_TMA) {
         if (lane == 0) {
             const int row0_3 = c0 - nc10 + toff3, row0_2 = c0 - nc10 + toff2;
@@ -470,9 +503,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             }
         }
     } else if (warp == WARP_MMA || warp == WARP_MMA2) {
-        // Two warps issue the MMAs, each into accumulators of its own (the first classes 0 and 1, the
-        // second class 2; on sweep 2 the two share class 3's sum between two accumulators), so no
-        // accumulator depends on the order of the two issuing threads.  One elected thread of each runs the
+        // Two warps issue the MMAs, each into accumulators of its own, so no accumulator depends on the
+        // order of the two issuing threads.  One elected thread of each runs the
         // whole loop: its operands are then uniform values for the compiler, which the shuffles say for
         // those that come from memory.  The B descriptors move with the start address alone (bits 0-13,
         // 16-byte units, no carry out for shared-memory addresses).
@@ -493,8 +525,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         t.flags = smem_u32(ab_flags);
         t.bars = smem_u32(ab_empty);
         const uint32_t tmem_u = uni((int)tmem);
-        t.acc = tmem_u + (second ? 2 * t.nmma : 0);
-        t.a_first = tmem_u + 3 * t.nmma;
+        t.acc = tmem_u + (second ? (FOUR ? 1 : 2) * t.nmma : 0);
+        t.a_first = tmem_u + ncls * t.nmma;
         t.ab = t.seen = t.s = t.ph = 0;
         t.need = 4;
         if (elect_one()) {
@@ -504,12 +536,17 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     // the epilogue of the previous item has read the accumulators out
                     ok = mbar_wait(acc_empty, (ni & 1) ^ 1, abort_flag, err, 32);
                     const int nsl = nslices(b);
-                    if (ok && sw == 0)
-                        ok = second ? issue_item<true, 0>(t, nsl, st_full, st_empty, abort_flag, err)
-                                    : issue_item<false, 0>(t, nsl, st_full, st_empty, abort_flag, err);
-                    else if (ok)
-                        ok = second ? issue_item<true, 1>(t, nsl, st_full, st_empty, abort_flag, err)
-                                    : issue_item<false, 1>(t, nsl, st_full, st_empty, abort_flag, err);
+                    if constexpr (FOUR) {
+                        if (ok)
+                            ok = second ? issue_item<true, SW_MASK4>(t, nsl, st_full, st_empty, abort_flag, err)
+                                        : issue_item<false, SW_MASK4>(t, nsl, st_full, st_empty, abort_flag, err);
+                    } else if (ok && sw == 0) {
+                        ok = second ? issue_item<true, SW_D>(t, nsl, st_full, st_empty, abort_flag, err)
+                                    : issue_item<false, SW_D>(t, nsl, st_full, st_empty, abort_flag, err);
+                    } else if (ok) {
+                        ok = second ? issue_item<true, SW_CLASS3>(t, nsl, st_full, st_empty, abort_flag, err)
+                                    : issue_item<false, SW_CLASS3>(t, nsl, st_full, st_empty, abort_flag, err);
+                    }
                     if (ok) umma_commit_bar(smem_u32(acc_full));
                 }
             if (!ok) {
@@ -552,9 +589,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         int s = 0, ph = 0, ni = 0, ab = ps % nabuf;
         int g = ps;               // next group of this set, counted from the current slice's first
         uint32_t abph = 1 ^ (ps / nabuf & 1);  // parity to wait for on ab_empty[ab]
-        auto form_slice = [&](auto ndc, auto onec) {
-            constexpr int ND = decltype(ndc)::value;
-            constexpr int D0 = ND - 3;                    // sweep 2 stores product digits 1-3
+        auto form_slice = [&](auto ndc, auto nsc, auto onec) {
+            constexpr int ND = decltype(ndc)::value, NS = decltype(nsc)::value;
+            constexpr int D0 = ND - NS;                   // ND digits formed, the last NS stored
             constexpr bool ONE = decltype(onec)::value;   // one anchor slot
             const uint32_t st = stage0 + (uint32_t)(s * st_bytes);
             for (; g < ngr; g += NSET) {
@@ -562,7 +599,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 asm volatile("ld.shared.b32 %0, [%1];" : "=r"(word) : "r"(group0 + 16 * g));
                 word = __shfl_sync(0xffffffffu, word, 0);
                 const uint32_t row = word & 0xffffu, blocks = word >> (16 + q);  // 16 × first row, live blocks
-                const uint32_t col = a_col0 + lane_field + ab * ABUF_COLS;
+                const uint32_t col = a_col0 + lane_field + ab * (NS == 4 ? ABUF4_COLS : ABUF_COLS);
                 // 16-byte chunk c of a 128-byte-swizzled row lies at chunk c ^ (row & 7)
                 auto chunk_of = [&](uint32_t r16) { return st + 8 * r16 + ((r16 & 0x70u) ^ c4); };
                 float4 v1[2];
@@ -576,7 +613,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 }
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {  // TMEM lanes 16·half .. +15 of the warp's 32
-                    uint32_t w[3][4];
+                    uint32_t w[NS][4];
 #pragma unroll
                     for (int jj = 0; jj < 2; ++jj) {
                         const int j = 2 * half + jj;
@@ -595,13 +632,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                                 digits254x2<ND>(make_float2(v1[h].x, v1[h].y), make_float2(x.x, x.y), ya);
                                 digits254x2<ND>(make_float2(v1[h].z, v1[h].w), make_float2(x.z, x.w), yb);
 #pragma unroll
-                                for (int dd = 0; dd < 3; ++dd)
+                                for (int dd = 0; dd < NS; ++dd)
                                     w[dd][2 * h + jj] =
                                         pack_low_bytes(ya[dd + D0].x, ya[dd + D0].y, yb[dd + D0].x, yb[dd + D0].y);
                             }
                         } else {
 #pragma unroll
-                            for (int dd = 0; dd < 3; ++dd) w[dd][jj] = w[dd][2 + jj] = 0u;
+                            for (int dd = 0; dd < NS; ++dd) w[dd][jj] = w[dd][2 + jj] = 0u;
                         }
                     }
                     if (half == 0) {
@@ -609,7 +646,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                         fence_after();
                     }
 #pragma unroll
-                    for (int dd = 0; dd < 3; ++dd) tmem_st16x8(col + ((uint32_t)(16 * half) << 16) + 8 * dd, w[dd]);
+                    for (int dd = 0; dd < NS; ++dd) tmem_st16x8(col + ((uint32_t)(16 * half) << 16) + 8 * dd, w[dd]);
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 fence_before();
@@ -625,13 +662,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             for (int sw = 0; sw < sweeps && ok; ++sw, ++ni) {
                 for (int sl = 0; sl < nslices(b); ++sl) {
                     if (!mbar_wait_conv(&st_ready[s], ph, abort_flag, err, 35)) { ok = false; break; }
-                    if (ks == 1) {
-                        if (sw == 0) form_slice(std::integral_constant<int, 3>(), std::true_type());
-                        else form_slice(std::integral_constant<int, 4>(), std::true_type());
-                    } else {
-                        if (sw == 0) form_slice(std::integral_constant<int, 3>(), std::false_type());
-                        else form_slice(std::integral_constant<int, 4>(), std::false_type());
-                    }
+                    auto form = [&](auto onec) {
+                        using std::integral_constant;
+                        if constexpr (FOUR) form_slice(integral_constant<int, 4>(), integral_constant<int, 4>(), onec);
+                        else if (sw == 0) form_slice(integral_constant<int, 3>(), integral_constant<int, 3>(), onec);
+                        else form_slice(integral_constant<int, 4>(), integral_constant<int, 3>(), onec);
+                    };
+                    if (ks == 1) form(std::true_type());
+                    else form(std::false_type());
                     if (!ok) break;
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&st_empty[s]);
@@ -641,26 +679,29 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 // ---- epilogue: int32 class accumulators → FP64, added into the unit's partial tile ----
                 if (!mbar_wait_warp(acc_full, ni & 1, abort_flag, err, 37)) { ok = false; break; }
                 fence_after();
-                const double scale = sw == 0 ? ldexp(1.0, E) * (1.0 / (16129.0 * 64516.0))
-                                             : ldexp(1.0, E) * (1.0 / (16129.0 * 16387064.0));
+                // one unit of the last class in the sums: 127^−2·254^−2 (classes 0-2) or 127^−2·254^−3
+                const double scale = ldexp(1.0, E) * (sw == 0 && !FOUR ? 1.0 / (16129.0 * 64516.0)
+                                                                       : 1.0 / (16129.0 * 16387064.0));
                 const bool first = b == u.b0 && sw == 0;
                 // this lane's accumulator row and anchor slot
                 const int r = row_of(32 * q + lane), a = ks > 1 ? r / rs : 0;
                 const bool row_ok = ks > 1 ? r < mrows && r - a * rs < nclen : r < mrows;
                 for (int cb = 8 * ps; cb < nmma; cb += 8 * NSET) {
-                    uint32_t v0[8], v1[8], v2[8];
+                    uint32_t v0[8], v1[8], v2[8], v3[8];
                     tmem_ld8(tmem + lane_field + cb, v0);
                     if (sw == 0) tmem_ld8(tmem + lane_field + nmma + cb, v1);
                     tmem_ld8(tmem + lane_field + 2 * nmma + cb, v2);
+                    if (FOUR) tmem_ld8(tmem + lane_field + 3 * nmma + cb, v3);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     if (!row_ok) continue;
 #pragma unroll
                     for (int e = 0; e < 8; ++e) {
                         const int colx = cb + e - a;  // slot a of a packed tile: lag column = column − a
                         if (colx < 0 || colx >= ncols) continue;
-                        const long long V = sw == 0 ? (long long)(int)v0[e] * 64516LL + (long long)(int)v1[e] * 254LL +
-                                                          (long long)(int)v2[e]
-                                                    : (long long)(int)v0[e] + (long long)(int)v2[e];
+                        long long V = (long long)(int)v0[e] + (long long)(int)v2[e];  // class 3 alone, in two parts
+                        if (sw == 0)
+                            V = (long long)(int)v0[e] * 64516LL + (long long)(int)v1[e] * 254LL + (long long)(int)v2[e];
+                        if (FOUR) V = V * 254LL + (long long)(int)v3[e];
                         double *o = out + (long)colx * LS_ROWS + r;
                         const double val = (double)V * scale;
                         *o = first ? val : *o + val;
@@ -717,34 +758,43 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
     if ((rc = ensure(c, c->misc, 256, "error flag"))) return rc;
     int *d_err = (int *)c->misc.p;
     if ((rc = cuda_check(c, cudaMemsetAsync(d_err, 0, sizeof(int), c->stream), "error flag"))) return rc;
-    constexpr size_t TILE_B = sizeof(double) * LS_ROWS * LS_ROWS;
     const size_t pcap = contract_partial_cap(c);
     const CUtensorMapDataType u8 = CU_TENSOR_MAP_DATA_TYPE_UINT8, f32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-    cudaFuncSetAttribute(ls_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+    cudaFuncSetAttribute(ls_i8_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+    cudaFuncSetAttribute(ls_i8_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
     size_t j0 = 0;
     while (j0 < jobs.size()) {
         // plan as many jobs as their partial tiles allow in one launch
         std::vector<LsJobPlan> plans;
-        long tiles = 0;
+        long used = 0;  // doubles of partial tiles
         size_t j1 = j0;
         for (; j1 < jobs.size(); ++j1) {
             const I8Job &jb = jobs[j1];
             LsJobPlan p;
             ls_plan_job(p, jb.nc, jb.nc10, jb.k, *jb.weight, c->num_sms, MIN_GROUPS, ls_force_bpu(c->chunk_px));
-            if (j1 > j0 && (size_t)(tiles + p.s.units()) * TILE_B > pcap) break;
-            p.unit_base = tiles;
-            tiles += p.s.units();
+            if (j1 > j0 && sizeof(double) * (size_t)(used + p.s.units() * p.s.tile()) > pcap) break;
+            p.unit_base = used;
+            used += p.s.units() * p.s.tile();
             plans.push_back(std::move(p));
         }
+        // the units of jobs that run in one four-class sweep, then the others: a launch each
         std::vector<LsUnit> units;
-        for (size_t i = 0; i < plans.size(); ++i) {
-            const size_t first = units.size();
-            ls_units(plans[i], (int)i, units);
-            if (jobs[j0 + i].mask_pass)
-                for (size_t q = first; q < units.size(); ++q) units[q].work *= 1.6;  // the class-3 sweep
+        size_t n4 = 0;
+        for (int four = 1; four >= 0; --four) {
+            const size_t begin = units.size();
+            for (size_t i = 0; i < plans.size(); ++i) {
+                const size_t first = units.size();
+                const bool mask = jobs[j0 + i].mask_pass;
+                if ((mask && mask4_fits(plans[i].s.cols(0))) != (four != 0)) continue;
+                ls_units(plans[i], (int)i, units);
+                if (mask && !four)
+                    for (size_t q = first; q < units.size(); ++q) units[q].work *= 1.6;  // the class-3 sweep
+            }
+            // largest units first, so that the small ones fill the tail of the launch
+            std::stable_sort(units.begin() + begin, units.end(),
+                             [](const LsUnit &a, const LsUnit &b) { return a.work > b.work; });
+            if (four) n4 = units.size();
         }
-        // largest units first, so that the small ones fill the tail of the launch
-        std::stable_sort(units.begin(), units.end(), [](const LsUnit &a, const LsUnit &b) { return a.work > b.work; });
         size_t ngroups = 0, noff = 0;
         for (const LsJobPlan &p : plans) {
             ngroups += p.groups.size();
@@ -754,7 +804,7 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
         const size_t off_u = (desc_b + 255) / 256 * 256, off_g = off_u + (unit_b + 255) / 256 * 256;
         const size_t off_o = off_g + (sizeof(int) * ngroups + 255) / 256 * 256;
         const size_t stage_b = off_o + sizeof(int) * noff;
-        if ((rc = ensure(c, c->partial, (size_t)tiles * TILE_B, "partial lag tiles"))) return rc;
+        if ((rc = ensure(c, c->partial, sizeof(double) * (size_t)used, "partial lag tiles"))) return rc;
         if ((rc = ensure(c, c->jobdesc, stage_b, "job list"))) return rc;
         // the staging area may still feed the previous launch's upload
         if ((rc = cuda_check(c, cudaStreamSynchronize(c->stream), "job staging"))) return rc;
@@ -800,7 +850,7 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
             x.rs = s.rs;
             x.AB = s.AB;
             x.T = s.T;
-            x.sweeps = jb.mask_pass ? 2 : 1;
+            x.mask = jb.mask_pass ? 1 : 0;
             x.tx_bytes = (uint32_t)(x.span3 * 128 + s.AB * 128 + 3 * 2 * x.span2 * 16);
             // whole 8-row swizzle atoms for the fp32 rows; every part starts on a 1024-byte boundary.  The
             // formers read a slot's whole 8-row blocks (all LS_ROWS rows with one slot) from every anchor on,
@@ -813,18 +863,24 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
             for (size_t q = 0; q < p.group_off.size(); ++q) ho[opos + q] = p.group_off[q];
             gpos += p.groups.size();
             opos += p.group_off.size();
-            red.push_back(LsReduceJob{(const double *)c->partial.p + p.unit_base * LS_ROWS * LS_ROWS, jb.lag_out,
-                                      s.nclen, s.k, s.rs, s.T, s.nab, s.V});
+            red.push_back(LsReduceJob{(const double *)c->partial.p + p.unit_base, jb.lag_out,
+                                      s.nclen, s.k, s.rs, s.T, s.nab, s.V, s.tile()});
         }
         std::copy(units.begin(), units.end(), (LsUnit *)(h + off_u));
         if ((rc = cuda_check(c, cudaMemcpyAsync(d, h, stage_b, cudaMemcpyHostToDevice, c->stream), "job list upload")))
             return rc;
         phase_begin(c, 1);
-        ls_i8_kernel<<<(unsigned)units.size(), NTHREADS, SMEM_BYTES, c->stream>>>(
-            (const I8Desc *)d, (const LsUnit *)(d + off_u), (double *)c->partial.p, d_err);
+        const LsUnit *du = (const LsUnit *)(d + off_u);
+        if (n4 > 0)
+            ls_i8_kernel<true><<<(unsigned)n4, NTHREADS, SMEM_BYTES, c->stream>>>((const I8Desc *)d, du,
+                                                                                 (double *)c->partial.p, d_err);
+        if (units.size() > n4)
+            ls_i8_kernel<false><<<(unsigned)(units.size() - n4), NTHREADS, SMEM_BYTES, c->stream>>>(
+                (const I8Desc *)d, du + n4, (double *)c->partial.p, d_err);
         phase_end(c);
-        c->launches += 1;
-        c->contractions += 1;
+        const int nl = (n4 > 0) + (units.size() > n4);
+        c->launches += nl;
+        c->contractions += nl;
         if ((rc = cuda_check(c, cudaGetLastError(), "ls_i8_kernel launch"))) return rc;
         if ((rc = ls_reduce(c, red))) return rc;
         j0 = j1;

@@ -25,7 +25,7 @@ __global__ void __launch_bounds__(32 * RED_PARTS) ls_reduce_kernel(const LsReduc
     const long ncsize = (long)j.nclen * j.nclen;
     const int lane = threadIdx.x, part = threadIdx.y;
     const long d = (long)blockIdx.x * 32 + lane;
-    constexpr long TILE = (long)LS_ROWS * LS_ROWS;
+    const long TILE = j.tile;
     double s = 0.0, comp = 0.0;
     auto add = [&](double v) {
         const double t = s + v, bp = t - s;
@@ -148,7 +148,7 @@ void ls_units(const LsJobPlan &p, int job, std::vector<LsUnit> &out)
                     u.ab = ab;
                     u.b0 = (int)(v * s.bpu);
                     u.b1 = (int)std::min(s.nblk, (v + 1) * s.bpu);
-                    u.tile = p.unit_base + local++;
+                    u.tile = p.unit_base + s.tile() * local++;
                     u.work = (double)(u.b1 - u.b0) * (p.group_off[ab + 1] - p.group_off[ab]);
                     out.push_back(u);
                 }

@@ -26,12 +26,13 @@
 // Work units.  The pixels are cut into blocks of LS_BLOCK; a unit is a tile
 // pair × an anchor block × a run of consecutive pixel blocks, run by one CTA,
 // which leaves the unit's FP64 sums in a partial tile of its own
-// [LS_ROWS][LS_ROWS].  ls_reduce then adds, per lag cell, the partial tiles of
+// [lag columns ≤ LS_ROWS][LS_ROWS].  ls_reduce then adds, per lag cell, the partial tiles of
 // every unit (and slot) in a fixed order with a compensated accumulator.  The
 // units of a job depend only on the job and the SM count, never on what else
 // shares the launch, so every result is deterministic.
 #pragma once
 
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -55,6 +56,7 @@ struct LsShape {
     int cols(int t2) const;  // MMA width N of tile t2 (multiple of 16)
     int lag_cols(int t2) const;  // lag columns Δ2 of tile t2 (k > 1: nclen)
     int units() const { return T * T * nab * V; }
+    long tile() const { return (long)LS_ROWS * std::min(LS_ROWS, nclen); }  // doubles of one partial tile
 };
 
 // min_groups: least work of a unit in anchor groups × pixel blocks, a block's own cost counted as two groups
@@ -71,7 +73,7 @@ struct LsUnit {
     short t3, t2;
     int ab;           // anchor block
     int b0, b1;       // pixel blocks [b0, b1)
-    long tile;        // its partial tile in the launch's partial buffer
+    long tile;        // its partial tile: doubles from the start of the launch's partial buffer
     double work;      // modelled cost (launch order: largest first)
 };
 
@@ -81,7 +83,7 @@ struct LsJobPlan {
     LsShape s;
     std::vector<int> groups;      // concatenated over anchor blocks
     std::vector<int> group_off;   // nab + 1 offsets into groups
-    long unit_base = 0;           // first partial tile of the job in its launch
+    long unit_base = 0;           // doubles before the job's first partial tile in its launch
 };
 void ls_plan_job(LsJobPlan &p, int nc, int nc10, long k_px, const std::vector<int> &weight, int sms,
                  long min_groups, long force_bpu = 0);
@@ -89,9 +91,10 @@ void ls_units(const LsJobPlan &p, int job, std::vector<LsUnit> &out);
 
 // Device description of one job for ls_reduce.
 struct LsReduceJob {
-    const double *partial;  // the job's partial tiles [units][LS_ROWS][LS_ROWS]
+    const double *partial;  // the job's partial tiles [units][lag columns][LS_ROWS]
     double *lag;            // FP64 lag array [nclen][nclen], row Δ2, column Δ3
     int nclen, k, rs, T, nab, V;
+    long tile;              // doubles of one partial tile
 };
 // lag = Σ over units (and slots) of the partial tiles, compensated, fixed order; one launch for
 // every job of a contraction launch.  The descriptors are copied into the context's job staging.
