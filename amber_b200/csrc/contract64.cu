@@ -39,7 +39,7 @@ struct F64Desc {
     const int *groups;           // anchor groups, concatenated over anchor blocks
     const int *group_off;        // [nab + 1]
     long k, kp;
-    int nc, nc10, nclen, ks, rs, AB;
+    int nc, nc10, nclen, ks, rs, ts, AB;
 };
 
 constexpr int F_S1 = LS_SPAN + 1;  // D1 rows of an anchor block (≤ 256)
@@ -79,13 +79,13 @@ __global__ void __launch_bounds__(F_NT, 1) ls_fp64_kernel(const F64Desc *__restr
     const int gq = lane >> 2, tq = lane & 3;   // fragment row / column group, k index
     const int ks = j.ks, nclen = j.nclen, nc = j.nc;
     const int c0 = u.ab * j.AB, c1 = min(nc, c0 + j.AB), nab1 = c1 - c0;
-    const int mrows = ks > 1 ? ks * j.rs : min(LS_ROWS, nclen - LS_ROWS * u.t3);
-    const int ncols = ks > 1 ? nclen + ks - 1 : min(LS_ROWS, nclen - LS_ROWS * u.t2);
-    const int row0_3 = c0 - j.nc10 + (ks > 1 ? 0 : LS_ROWS * u.t3);  // channel of staged D3 row 0
-    const int row0_2 = c0 - j.nc10 + (ks > 1 ? 0 : LS_ROWS * u.t2);  // channel of staged D2 row 0
+    const int mrows = ks > 1 ? ks * j.rs : min(j.ts, nclen - j.ts * u.t3);
+    const int ncols = ks > 1 ? nclen + ks - 1 : min(j.ts, nclen - j.ts * u.t2);
+    const int row0_3 = c0 - j.nc10 + (ks > 1 ? 0 : j.ts * u.t3);  // channel of staged D3 row 0
+    const int row0_2 = c0 - j.nc10 + (ks > 1 ? 0 : j.ts * u.t2);  // channel of staged D2 row 0
     const int span3 = nab1 + (ks > 1 ? nclen : mrows) - 1;
     const int span2 = nab1 + ncols - 1;
-    const int toff3 = ks > 1 ? 0 : LS_ROWS * u.t3, toff2 = ks > 1 ? 0 : LS_ROWS * u.t2;
+    const int toff3 = ks > 1 ? 0 : j.ts * u.t3, toff2 = ks > 1 ? 0 : j.ts * u.t2;
     // The unit's anchor groups {first channel, live column fragments (bits 0-15) and row fragments (bits
     // 16-23)}: fragments whose D2 or D3 channels all lie outside [0, nc) add only zeros and are skipped, and
     // a group without a live fragment (a corner tile of a wide window) is dropped.
@@ -390,13 +390,13 @@ int contract_fp64_jobs(amber_cuda_ctx *c, const std::vector<F64Job> &jobs)
             x.groups = (const int *)(d + off_g) + gpos;
             x.group_off = (const int *)(d + off_o) + opos;
             x.k = jb.k; x.kp = jb.kp;
-            x.nc = (int)c->nc; x.nc10 = c->nc10; x.nclen = nclen; x.ks = p.s.k; x.rs = p.s.rs; x.AB = p.s.AB;
+            x.nc = (int)c->nc; x.nc10 = c->nc10; x.nclen = nclen; x.ks = p.s.k; x.rs = p.s.rs; x.ts = p.s.ts; x.AB = p.s.AB;
             std::copy(p.groups.begin(), p.groups.end(), hg + gpos);
             for (size_t q = 0; q < p.group_off.size(); ++q) ho[opos + q] = p.group_off[q];
             gpos += p.groups.size();
             opos += p.group_off.size();
             red.push_back(LsReduceJob{(const double *)c->partial.p + p.unit_base, jb.lag_out, nclen,
-                                      p.s.k, p.s.rs, p.s.T, p.s.nab, p.s.V, p.s.tile()});
+                                      p.s.k, p.s.rs, p.s.T, p.s.ts, p.s.nab, p.s.V, p.s.tile()});
         }
         std::copy(units.begin(), units.end(), (LsUnit *)(h + off_u));
         if ((rc = cuda_check(c, cudaMemcpyAsync(d, h, stage_b, cudaMemcpyHostToDevice, c->stream), "job list upload")))

@@ -27,8 +27,8 @@
 // 4.5e-8 (mask, classes 0-3), against 5–8e-7 for the mask maps without class 3.
 // A per-block exponent is what lets all anchors share one accumulator: the
 // scale of a product no longer depends on its channels.  |class sum| ≤
-// 3·127² per pixel and anchor, and a block holds at most 128 anchor groups of
-// 256 pixels (32768 terms): the int32 accumulators cannot overflow.
+// 3·127² per pixel and anchor, and a block holds at most 173 anchor groups of
+// 256 pixels (44288 terms): the int32 accumulators cannot overflow.
 //
 // Operands.  A (TMEM, M = 128 rows Δ3, written by the formers with tcgen05.st)
 // = the per-anchor product digits; B (shared memory, N ≤ 128 rows Δ2) = the D2
@@ -113,7 +113,7 @@ struct alignas(64) I8Desc {
     const int *e1, *e2, *e3;        // block exponents
     const int *groups, *group_off;  // anchor groups of every anchor block
     long k;
-    int nc, nc10, nclen, ks, rs, AB, T;
+    int nc, nc10, nclen, ks, rs, AB, ts;
     int span3, span2;
     int mask;                       // sampling-mask maps: class 3 as well
     uint32_t tx_bytes;              // bytes one slice's three TMA boxes deliver
@@ -368,9 +368,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     const I8Desc *jd = jobs + u.job;
     const int ks = jd->ks, nclen = jd->nclen, nc = jd->nc, nc10 = jd->nc10, rs = jd->rs;
     const int c0 = u.ab * jd->AB, c1 = min(nc, c0 + jd->AB);
-    const int toff3 = ks > 1 ? 0 : LS_ROWS * u.t3, toff2 = ks > 1 ? 0 : LS_ROWS * u.t2;
-    const int mrows = ks > 1 ? ks * rs : min(LS_ROWS, nclen - toff3);
-    const int ncols = ks > 1 ? nclen : min(LS_ROWS, nclen - toff2);  // lag columns
+    const int ts = jd->ts, toff3 = ks > 1 ? 0 : ts * u.t3, toff2 = ks > 1 ? 0 : ts * u.t2;
+    const int mrows = ks > 1 ? ks * rs : min(ts, nclen - toff3);
+    const int ncols = ks > 1 ? nclen : min(ts, nclen - toff2);  // lag columns
     const int nwin = ks > 1 ? nclen + ks - 1 : ncols;                // window rows of D2
     const int nmma = ((nwin + 15) / 16) * 16;                        // MMA N
     // Sweeps of an item: classes 0-2 alone (SW_D); for the mask maps all four classes at once where four
@@ -849,7 +849,7 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
             x.ks = s.k;
             x.rs = s.rs;
             x.AB = s.AB;
-            x.T = s.T;
+            x.ts = s.ts;
             x.mask = jb.mask_pass ? 1 : 0;
             x.tx_bytes = (uint32_t)(x.span3 * 128 + s.AB * 128 + 3 * 2 * x.span2 * 16);
             // whole 8-row swizzle atoms for the fp32 rows; every part starts on a 1024-byte boundary.  The
@@ -864,7 +864,7 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
             gpos += p.groups.size();
             opos += p.group_off.size();
             red.push_back(LsReduceJob{(const double *)c->partial.p + p.unit_base, jb.lag_out,
-                                      s.nclen, s.k, s.rs, s.T, s.nab, s.V, s.tile()});
+                                      s.nclen, s.k, s.rs, s.T, s.ts, s.nab, s.V, s.tile()});
         }
         std::copy(units.begin(), units.end(), (LsUnit *)(h + off_u));
         if ((rc = cuda_check(c, cudaMemcpyAsync(d, h, stage_b, cudaMemcpyHostToDevice, c->stream), "job list upload")))

@@ -41,8 +41,8 @@ __global__ void __launch_bounds__(32 * RED_PARTS) ls_reduce_kernel(const LsReduc
         if (j.k > 1) {
             p = j.partial + (long)d2 * LS_ROWS + d3;
         } else {
-            const int t2 = d2 / LS_ROWS, t3 = d3 / LS_ROWS;
-            p = j.partial + (long)(t3 * j.T + t2) * j.nab * j.V * TILE + (long)(d2 % LS_ROWS) * LS_ROWS + d3 % LS_ROWS;
+            const int t2 = d2 / j.ts, t3 = d3 / j.ts;
+            p = j.partial + (long)(t3 * j.T + t2) * j.nab * j.V * TILE + (long)(d2 % j.ts) * LS_ROWS + d3 % j.ts;
         }
         p += (i0 / j.k) * TILE + (i0 % j.k) * j.rs;
         int slot = i0 % j.k;
@@ -78,12 +78,12 @@ __global__ void __launch_bounds__(32 * RED_PARTS) ls_reduce_kernel(const LsReduc
 
 }  // namespace
 
-int LsShape::rows(int t3) const { return k > 1 ? k * rs : std::min(LS_ROWS, nclen - LS_ROWS * t3); }
+int LsShape::rows(int t3) const { return k > 1 ? k * rs : std::min(ts, nclen - ts * t3); }
 int LsShape::cols(int t2) const
 {
-    return k > 1 ? round16(nclen + k - 1) : round16(std::min(LS_ROWS, nclen - LS_ROWS * t2));
+    return k > 1 ? round16(nclen + k - 1) : round16(std::min(ts, nclen - ts * t2));
 }
-int LsShape::lag_cols(int t2) const { return k > 1 ? nclen : std::min(LS_ROWS, nclen - LS_ROWS * t2); }
+int LsShape::lag_cols(int t2) const { return k > 1 ? nclen : std::min(ts, nclen - ts * t2); }
 
 LsShape ls_shape(int nc, int nc10, long k_px, int sms, long min_groups, long force_bpu)
 {
@@ -94,12 +94,18 @@ LsShape ls_shape(int nc, int nc10, long k_px, int sms, long min_groups, long for
     s.rs = (s.nclen + 7) / 8 * 8;
     s.k = s.rs <= LS_ROWS / 2 ? LS_ROWS / s.rs : 1;
     s.T = s.k > 1 ? 1 : (s.nclen + LS_ROWS - 1) / LS_ROWS;
+    // Near-equal tiles of whole 8-row blocks: an edge tile of a few lags costs nearly a whole one (an MMA at
+    // least 42 cycles, the formers all its rows against one column), so 129 lags run as 72 + 57.
+    s.ts = std::min(LS_ROWS, ((s.nclen + s.T - 1) / s.T + 7) / 8 * 8);
     // Staged rows of one unit: D3 spans AB + rows − 1 channels and the D2 window AB + N − 1;
-    // both must fit one TMA box (LS_SPAN rows).  An anchor block also holds at most 128 anchor
-    // groups, so that 128 groups × LS_BLOCK pixels of int8 digit products cannot overflow the
-    // int32 accumulators (|class sum| ≤ 3·127² per term, 32768 terms < 2^31 / 48387).
+    // both must fit one TMA box (LS_SPAN rows).  An anchor block also holds at most LS_GROUPS anchor
+    // groups, so that they and LS_BLOCK pixels of int8 digit products cannot overflow the int32 accumulators
+    // (|class sum| ≤ 3·127² per term, 2^31 / 48387 = 44381 terms).  The channels go into blocks of equal
+    // size: a last block of a few anchors would pay a whole unit's staging.
     const int span_extra = std::max(s.rows(0), s.cols(0)) - 1;
-    s.AB = std::max(1, std::min({nc, LS_SPAN - span_extra, LS_ROWS * s.k}));
+    const int widest = std::max(1, std::min({nc, LS_SPAN - span_extra, LS_GROUPS * s.k}));
+    s.nab = (nc + widest - 1) / widest;
+    s.AB = std::min(widest, ((nc + s.nab - 1) / s.nab + s.k - 1) / s.k * s.k);
     s.nab = (nc + s.AB - 1) / s.AB;
     s.nblk = std::max<long>(1, (k_px + LS_BLOCK - 1) / LS_BLOCK);
     // Units: about six per SM for a large job, so the last wave is short; each of at least min_groups

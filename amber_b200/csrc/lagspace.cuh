@@ -21,7 +21,8 @@
 // tile, rs being nclen rounded up to a multiple of 8 (so that an 8-row block
 // belongs to one anchor): row r = a·rs + Δ3 holds anchor slot a, and B is the
 // window of the first anchor widened to N = nclen + k − 1 rows, so slot a's lag
-// is Δ2 = column − a.  Large windows (nclen > 128) use ⌈nclen/128⌉² tile pairs.
+// is Δ2 = column − a.  Large windows (nclen > 128) use T² pairs of near-equal
+// tiles, T = ⌈nclen/128⌉.
 //
 // Work units.  The pixels are cut into blocks of LS_BLOCK; a unit is a tile
 // pair × an anchor block × a run of consecutive pixel blocks, run by one CTA,
@@ -42,12 +43,13 @@ namespace amber {
 constexpr int LS_BLOCK = 256;  // pixels per block (the int8 path's exponent block)
 constexpr int LS_ROWS = 128;   // accumulator rows and columns of one tile
 constexpr int LS_SPAN = 256;   // most channel rows one unit stages (a TMA box height)
+constexpr int LS_GROUPS = 173; // most anchor groups of one anchor block (int32 accumulators of the int8 path)
 
 struct LsShape {
     int nc, nc10, nclen;
     int k;        // anchor slots per tile (1 unless nclen ≤ 64)
     int rs;       // rows from one anchor slot to the next: nclen rounded up to whole 8-row blocks
-    int T;        // tiles per lag axis
+    int T, ts;    // tiles per lag axis, lags per tile (one slot): the axis in T near-equal parts
     int AB, nab;  // anchor-block width in channels, number of anchor blocks
     long nblk;    // pixel blocks
     long bpu;     // pixel blocks per unit
@@ -56,7 +58,7 @@ struct LsShape {
     int cols(int t2) const;  // MMA width N of tile t2 (multiple of 16)
     int lag_cols(int t2) const;  // lag columns Δ2 of tile t2 (k > 1: nclen)
     int units() const { return T * T * nab * V; }
-    long tile() const { return (long)LS_ROWS * std::min(LS_ROWS, nclen); }  // doubles of one partial tile
+    long tile() const { return (long)LS_ROWS * std::min(ts, nclen); }  // doubles of one partial tile
 };
 
 // min_groups: least work of a unit in anchor groups × pixel blocks, a block's own cost counted as two groups
@@ -93,7 +95,7 @@ void ls_units(const LsJobPlan &p, int job, std::vector<LsUnit> &out);
 struct LsReduceJob {
     const double *partial;  // the job's partial tiles [units][lag columns][LS_ROWS]
     double *lag;            // FP64 lag array [nclen][nclen], row Δ2, column Δ3
-    int nclen, k, rs, T, nab, V;
+    int nclen, k, rs, T, ts, nab, V;
     long tile;              // doubles of one partial tile
 };
 // lag = Σ over units (and slots) of the partial tiles, compensated, fixed order; one launch for

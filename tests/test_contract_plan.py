@@ -16,7 +16,8 @@ WINDOWS = [
     (33, 31, [0, 32]),     # nclen 63: two slots of 64 rows
     (34, 32, None),        # nclen 65: one slot, the first past the packed tiles
     (48, 47, [5]),         # nclen 95: N = 96
-    (66, 64, None),        # nclen 129: two tiles an axis, the second one row high
+    (66, 64, None),        # nclen 129: two tiles an axis, 72 + 57 lags
+    (150, 63, [140]),      # nclen 127, 150 channels: two anchor blocks of 75
 ]
 
 
