@@ -410,7 +410,7 @@ class Estimator:
                                                           np.float32(nu_chan0), int(flag_key), g, npar, nstokes,
                                                           _ptr(randpar, _fp), _ptr(data, _fp), int(n_collapse),
                                                           _ptr(ri, _dp), _ptr(nt, _dp)))
-        return ri[..., 0] + 1j * ri[..., 1], nt
+        return ri.view(np.complex128)[..., 0], nt
 
 
 def _request_of(real, want_v2, cyl=None, with_cube=True):

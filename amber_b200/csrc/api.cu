@@ -74,6 +74,11 @@ static void release(amber_cuda_ctx *c, DevBuf &b)
 
 int twiddle_table(amber_cuda_ctx *c, long n, const double2 **out)
 {
+    if (c->tw_owner) {
+        const int rc = twiddle_table(c->tw_owner, n, out);
+        if (rc) c->err = c->tw_owner->err;
+        return rc;
+    }
     auto it = c->twiddles.find(n);
     if (it == c->twiddles.end()) {
         std::vector<double2> h(n);
@@ -93,6 +98,32 @@ int twiddle_table(amber_cuda_ctx *c, long n, const double2 **out)
     }
     *out = reinterpret_cast<const double2 *>(it->second.p);
     return AMBER_OK;
+}
+
+int job_stage(amber_cuda_ctx *c, size_t bytes, void **host)
+{
+    int rc;
+    c->stage_i ^= 1;
+    amber_cuda_ctx::Stage &s = c->stage[c->stage_i];
+    if (s.sent) {
+        if ((rc = cuda_check(c, cudaEventSynchronize(s.sent), "job staging"))) return rc;
+    } else if ((rc = cuda_check(c, cudaEventCreateWithFlags(&s.sent, cudaEventDisableTiming), "job staging"))) {
+        return rc;
+    }
+    if (s.bytes < bytes) {
+        if (s.p) cudaFreeHost(s.p);
+        s.p = nullptr;
+        s.bytes = 0;
+        if ((rc = cuda_check(c, cudaHostAlloc(&s.p, bytes + bytes / 2, cudaHostAllocDefault), "job staging"))) return rc;
+        s.bytes = bytes + bytes / 2;
+    }
+    *host = s.p;
+    return AMBER_OK;
+}
+
+int job_stage_sent(amber_cuda_ctx *c)
+{
+    return cuda_check(c, cudaEventRecord(c->stage[c->stage_i].sent, c->stream), "job staging");
 }
 
 void phase_begin(amber_cuda_ctx *c, int phase)
@@ -228,6 +259,22 @@ std::vector<int> closed_triangles(const std::vector<double> &ulow, const std::ve
 
 // ---- one realisation's triangles, run in map-set batches ----
 
+// Device bytes of one ring slot of one map set (D or mask).
+static size_t slot_bytes(int precision, long ng, long nc)
+{
+    const size_t vbytes = precision == AMBER_PREC_FP64 ? 8 : (precision == AMBER_PREC_MIXED ? 7 : 4);
+    const long kalign = precision == AMBER_PREC_MIXED ? LS_BLOCK : 64;
+    const long kp = (ng * ng + kalign - 1) / kalign * kalign;
+    return vbytes * (size_t)nc * kp + 8 * (size_t)nc + 4 * (size_t)(kp / LS_BLOCK + 1);
+}
+
+// Bytes the maps leave free: the mixed-precision contraction's partial tiles when they live in this context.
+static size_t map_reserve(const amber_cuda_ctx *c)
+{
+    return ((size_t)64 << 20) +
+           (c->precision == AMBER_PREC_MIXED && !c->contracts_elsewhere ? contract_partial_cap(c) : 0);
+}
+
 int run_begin(amber_cuda_ctx *c, RunState &st, int ntri, const int *tri, int want_v2)
 {
     if (!c || ntri < 0 || (ntri > 0 && !tri)) return AMBER_ERR_ARG;
@@ -256,15 +303,31 @@ int run_begin(amber_cuda_ctx *c, RunState &st, int ntri, const int *tri, int wan
         }
         it->tris.push_back(t);
     }
+    // The maps of the largest group at once, where the budget holds them: grown group by group they would be
+    // freed and allocated again for each.
+    size_t maps = 0, y = 0;
+    const int passes = want_v2 ? 2 : 1;
+    for (const RunState::Group &g : st.groups) {
+        std::set<int> rings;
+        for (int t : g.tris) rings.insert(tri + 3 * t, tri + 3 * t + 3);
+        long jmax = 1;
+        for (int r : rings) jmax = std::max(jmax, std::min(g.ng / 3, (long)ceil(c->uhigh[r])));
+        maps = std::max(maps, slot_bytes(c->precision, g.ng, c->nc) * rings.size());
+        y = std::max(y, sizeof(double2) * rings.size() * (size_t)g.ng * jmax * c->nc);
+    }
+    const size_t other = c->held - c->maps_d.bytes - c->maps_i.bytes - c->y.bytes;
+    if (other + passes * std::max(maps, std::max(c->maps_d.bytes, c->maps_i.bytes)) + std::max(y, c->y.bytes) +
+            map_reserve(c) <= c->budget) {
+        if ((rc = ensure(c, c->maps_d, maps, "ring maps"))) return rc;
+        if (want_v2 && (rc = ensure(c, c->maps_i, maps, "ring mask maps"))) return rc;
+        if ((rc = ensure(c, c->y, y, "map intermediate"))) return rc;
+    }
     return AMBER_OK;
 }
 
 size_t map_slot_bytes(int precision, long ng, long nc, int want_v2)
 {
-    const size_t vbytes = precision == AMBER_PREC_FP64 ? 8 : (precision == AMBER_PREC_MIXED ? 7 : 4);
-    const long kalign = precision == AMBER_PREC_MIXED ? LS_BLOCK : 64;
-    const long k = ng * ng, kp = (k + kalign - 1) / kalign * kalign;
-    const size_t per_pass = vbytes * (size_t)nc * kp + 8 * (size_t)nc + 4 * (size_t)(kp / LS_BLOCK + 1);
+    const size_t per_pass = slot_bytes(precision, ng, nc);
     // + the map builder's column-pass intermediate (double2 per ring row, column and channel)
     const size_t y = sizeof(double2) * (size_t)ng * (size_t)(ng / 3 + 1) * (size_t)nc;
     return per_pass * (want_v2 ? 2 : 1) + y;
@@ -285,20 +348,17 @@ int run_next_batch(amber_cuda_ctx *c, RunState &st, std::vector<I8Job> *jobs)
     const int nclen = 2 * c->nc10 + 1;
     const long ncsize = (long)nclen * nclen;
     double *res = (double *)c->results.p;
-    const size_t vbytes = prec == AMBER_PREC_FP64 ? 8 : (prec == AMBER_PREC_MIXED ? 7 : 4);
     const long kalign = prec == AMBER_PREC_MIXED ? LS_BLOCK : 64;
     const long k = g.ng * g.ng, kp = (k + kalign - 1) / kalign * kalign;
     const long nblk = kp / LS_BLOCK;
-    const size_t per_slot = vbytes * (size_t)c->nc * kp + 8 * (size_t)c->nc + 4 * (size_t)(nblk + 1);
+    const size_t per_slot = slot_bytes(prec, g.ng, c->nc);
     // The next batch of the group: triangles whose ring union fits the budget.
     size_t spare = c->budget > c->held ? c->budget - c->held : 0;
     spare += c->maps_d.bytes + c->maps_i.bytes + c->y.bytes;
     // the partial tiles of the last contraction give way to maps: the mixed path's reserve below covers
     // them, the FP64 path frees them when the maps need the room and takes what is left afterwards
     if (!c->contracts_elsewhere) spare += c->partial.bytes;
-    // keep room for the mixed-precision contraction's partial tiles when they live in this context
-    const size_t reserve = ((size_t)64 << 20) +
-                           (prec == AMBER_PREC_MIXED && !c->contracts_elsewhere ? contract_partial_cap(c) : 0);
+    const size_t reserve = map_reserve(c);
     const long cap_slots = (long)((spare > reserve ? spare - reserve : 0) /
                                   (map_slot_bytes(prec, g.ng, c->nc, want_v2) + 1));
     if (cap_slots < 3) return fail(c, AMBER_ERR_OOM, "maps of one triangle (Ng1=%ld) exceed the budget", g.ng);
@@ -390,7 +450,7 @@ int run_next_batch(amber_cuda_ctx *c, RunState &st, std::vector<I8Job> *jobs)
         const size_t ss = (size_t)c->nc * kp;
         for (int pass = 0; pass < (want_v2 ? 2 : 1); ++pass) {
             void *base = pass == 0 ? c->maps_d.p : c->maps_i.p;
-            double *lag = res + ((size_t)t * 2 + pass) * ncsize;
+            double *lag = res + ((size_t)pass * (st.tri.size() / 3) + t) * ncsize;
             if (prec == AMBER_PREC_MIXED) {
                 const DigitMaps &b = dmaps[pass];
                 auto slot = [&](size_t s) {
@@ -423,9 +483,26 @@ int run_next_batch(amber_cuda_ctx *c, RunState &st, std::vector<I8Job> *jobs)
         }
         c->last_products += (double)c->total_vcp * (double)k * (want_v2 ? 2.0 : 1.0);
     }
-    if (!local.empty() && (rc = contract_i8_jobs(c, local))) return rc;
+    if (!local.empty() && ((rc = contract_i8_jobs(c, local)) || (rc = contract_i8_finish(c)))) return rc;
     if (!f64jobs.empty() && (rc = contract_fp64_jobs(c, f64jobs))) return rc;
     return 1;
+}
+
+amber_cuda_ctx *child_context(amber_cuda_ctx *owner, size_t budget)
+{
+    amber_cuda_ctx *c = new amber_cuda_ctx();
+    c->device = owner->device;
+    c->precision = owner->precision;
+    c->fp64_abs = owner->fp64_abs;
+    c->chunk_px = owner->chunk_px;
+    c->num_sms = owner->num_sms;
+    c->stream = owner->stream;
+    c->budget = budget;
+    c->tw_owner = owner;
+    c->contracts_elsewhere = owner->precision == AMBER_PREC_MIXED;
+    cudaEventCreate(&c->ev0);
+    cudaEventCreate(&c->ev1);
+    return c;
 }
 
 }  // namespace amber
@@ -497,8 +574,10 @@ void amber_cuda_destroy(amber_cuda_ctx *c)
     DevBuf *bufs[] = {&c->grid, &c->mask, &c->d_weight, &c->d_anchors, &c->y, &c->maps_d, &c->maps_i,
                       &c->partial, &c->results, &c->ring_lohi, &c->misc, &c->mixed_scratch, &c->lagred, &c->jobdesc, &c->lagtrial, &c->lsred};
     for (DevBuf *b : bufs) release(c, *b);
-    if (c->stage) cudaFreeHost(c->stage);
-    c->stage = nullptr;
+    for (amber_cuda_ctx::Stage &s : c->stage) {
+        if (s.p) cudaFreeHost(s.p);
+        if (s.sent) cudaEventDestroy(s.sent);
+    }
     for (auto &kv : c->twiddles) release(c, kv.second);
     for (auto &e : c->phase_ev) {
         cudaEventDestroy(e.a);
@@ -707,6 +786,7 @@ int amber_cuda_triangles_run(amber_cuda_ctx *c, int ntri, const int *tri, int wa
     c->phase_used = 0;
     c->launches = 0;
     c->contractions = 0;
+    c->i8_open = false;
     cudaEventRecord(c->ev0, c->stream);
     const bool mixed = c->precision == AMBER_PREC_MIXED;
     std::vector<amber::I8Job> jobs;
@@ -717,6 +797,7 @@ int amber_cuda_triangles_run(amber_cuda_ctx *c, int ntri, const int *tri, int wa
     }
     if (rc < 0) return rc;
     cudaEventRecord(c->ev1, c->stream);
+    if (mixed && (rc = amber::contract_i8_finish(c))) return rc;
     if ((rc = cuda_check(c, cudaEventSynchronize(c->ev1), "triangle run"))) return rc;
     if ((rc = cuda_check(c, cudaGetLastError(), "triangle run"))) return rc;
     cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1);
@@ -739,20 +820,18 @@ int amber_cuda_triangles_fetch(amber_cuda_ctx *c, double *bldnu, int64_t *numdnu
     const int n = c->last_ntri;
     int rc;
     cudaSetDevice(c->device);
-    for (int t = 0; t < n; ++t) {
-        const double *src = (const double *)c->results.p + (size_t)t * 2 * ncsize;
-        if (bldnu &&
-            (rc = cuda_check(c, cudaMemcpyAsync(bldnu + (size_t)t * ncsize, src, sizeof(double) * ncsize,
-                                                cudaMemcpyDeviceToHost, c->stream),
-                             "fetch bldnu")))
-            return rc;
-        if (numtri && c->last_v2 &&
-            (rc = cuda_check(c, cudaMemcpyAsync(numtri + (size_t)t * ncsize, src + ncsize, sizeof(double) * ncsize,
-                                                cudaMemcpyDeviceToHost, c->stream),
-                             "fetch numtri")))
-            return rc;
-        if (numdnu) memcpy(numdnu + (size_t)t * ncsize, c->counts.data(), sizeof(int64_t) * ncsize);
-    }
+    const double *src = (const double *)c->results.p;
+    const size_t bytes = sizeof(double) * (size_t)ncsize * n;
+    if (n > 0 && bldnu &&
+        (rc = cuda_check(c, cudaMemcpyAsync(bldnu, src, bytes, cudaMemcpyDeviceToHost, c->stream), "fetch bldnu")))
+        return rc;
+    if (n > 0 && numtri && c->last_v2 &&
+        (rc = cuda_check(c, cudaMemcpyAsync(numtri, src + (size_t)ncsize * n, bytes, cudaMemcpyDeviceToHost, c->stream),
+                         "fetch numtri")))
+        return rc;
+    if (numdnu)
+        for (int t = 0; t < n; ++t)
+            memcpy(numdnu + (size_t)t * ncsize, c->counts.data(), sizeof(int64_t) * ncsize);
     return cuda_check(c, cudaStreamSynchronize(c->stream), "fetch");
 }
 

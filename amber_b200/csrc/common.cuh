@@ -76,7 +76,7 @@ struct amber_cuda_ctx {
     amber::DevBuf maps_d;   // D maps (FP64 path: double; mixed path: split planes)
     amber::DevBuf maps_i;   // I maps (v2)
     amber::DevBuf partial;  // per-anchor/k-split partial lag tiles
-    amber::DevBuf results;  // per-triangle FP64 lag arrays [ntri][2][nclen²]
+    amber::DevBuf results;  // FP64 lag arrays [2][ntri][nclen²]: D sums, then mask sums
     amber::DevBuf ring_lohi;
     amber::DevBuf misc;
     amber::DevBuf mixed_scratch;
@@ -84,8 +84,16 @@ struct amber_cuda_ctx {
     amber::DevBuf jobdesc; // contraction job descriptors and work items
     amber::DevBuf lagtrial; // autotuner: lag array of a discarded trial run
     amber::DevBuf lsred;    // lag-space reduction: job descriptors
-    void *stage = nullptr; // pinned host staging of the job descriptors
-    size_t stage_bytes = 0;
+    // pinned host staging of the job descriptors: two in turn, so that a launch is prepared while the upload
+    // of the one before is still to run
+    struct Stage {
+        void *p = nullptr;
+        size_t bytes = 0;
+        cudaEvent_t sent = nullptr;  // recorded after the upload from p
+    } stage[2];
+    int stage_i = 0;
+    bool i8_open = false;  // int8 contractions launched whose error flag has not been read
+    amber_cuda_ctx *tw_owner = nullptr;  // an engine's child context: the owner keeps the twiddle tables
     amber::Engine *engine = nullptr;  // batched requests, created on the first enqueue
     bool contracts_elsewhere = false; // an engine's child context: its jobs run in the owner's contraction
 
@@ -120,6 +128,10 @@ int fail(amber_cuda_ctx *c, int code, const char *fmt, ...);
 int cuda_check(amber_cuda_ctx *c, cudaError_t e, const char *what);
 int ensure(amber_cuda_ctx *c, DevBuf &b, size_t bytes, const char *what);
 int twiddle_table(amber_cuda_ctx *c, long n, const double2 **out);
+// The next pinned staging buffer, free to write (waits for its last upload); job_stage_sent after enqueuing the
+// upload from it.
+int job_stage(amber_cuda_ctx *c, size_t bytes, void **host);
+int job_stage_sent(amber_cuda_ctx *c);
 
 // Map builder: ring-mask + unnormalised c2r of every channel of the given
 // rings onto an ng × ng grid.  src_complex: double2 grid; else real mask.
@@ -179,7 +191,11 @@ struct I8Job {
 };
 // All jobs in as few persistent launches as the partial-tile memory allows (jobs of
 // different realisations may share a launch); each job's result depends on the job only.
+// Enqueues only: contract_i8_finish waits for the stream and reads the error flag of all calls since the last.
 int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs);
+int contract_i8_finish(amber_cuda_ctx *c);
+// A context of an engine's request: the owner's device, options and stream, its own budget.
+amber_cuda_ctx *child_context(amber_cuda_ctx *owner, size_t budget);
 
 // One realisation's list of triangles, run in map-set batches: the triangles are grouped
 // by r1 (one Ng1 grid per group) and each group is cut into batches whose ring maps fit

@@ -368,15 +368,9 @@ int contract_fp64_jobs(amber_cuda_ctx *c, const std::vector<F64Job> &jobs)
         const size_t stage_b = off_o + sizeof(int) * noff;
         if ((rc = ensure(c, c->partial, sizeof(double) * (size_t)used, "partial lag tiles"))) return rc;
         if ((rc = ensure(c, c->jobdesc, stage_b, "job list"))) return rc;
-        if ((rc = cuda_check(c, cudaStreamSynchronize(c->stream), "job staging"))) return rc;
-        if (c->stage_bytes < stage_b) {
-            if (c->stage) cudaFreeHost(c->stage);
-            c->stage = nullptr;
-            c->stage_bytes = 0;
-            if ((rc = cuda_check(c, cudaHostAlloc(&c->stage, stage_b, cudaHostAllocDefault), "job staging"))) return rc;
-            c->stage_bytes = stage_b;
-        }
-        char *h = (char *)c->stage, *d = (char *)c->jobdesc.p;
+        void *staging;
+        if ((rc = job_stage(c, stage_b, &staging))) return rc;
+        char *h = (char *)staging, *d = (char *)c->jobdesc.p;
         F64Desc *hd = (F64Desc *)h;
         int *hg = (int *)(h + off_g), *ho = (int *)(h + off_o);
         std::vector<LsReduceJob> red;
@@ -401,6 +395,7 @@ int contract_fp64_jobs(amber_cuda_ctx *c, const std::vector<F64Job> &jobs)
         std::copy(units.begin(), units.end(), (LsUnit *)(h + off_u));
         if ((rc = cuda_check(c, cudaMemcpyAsync(d, h, stage_b, cudaMemcpyHostToDevice, c->stream), "job list upload")))
             return rc;
+        if ((rc = job_stage_sent(c))) return rc;
         cudaFuncSetAttribute(ls_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F_SMEM);
         phase_begin(c, 1);
         for (size_t u0 = 0; u0 < units.size(); u0 += 1u << 30) {

@@ -757,7 +757,8 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
     if (jobs.empty()) return AMBER_OK;
     if ((rc = ensure(c, c->misc, 256, "error flag"))) return rc;
     int *d_err = (int *)c->misc.p;
-    if ((rc = cuda_check(c, cudaMemsetAsync(d_err, 0, sizeof(int), c->stream), "error flag"))) return rc;
+    if (!c->i8_open && (rc = cuda_check(c, cudaMemsetAsync(d_err, 0, sizeof(int), c->stream), "error flag"))) return rc;
+    c->i8_open = true;
     const size_t pcap = contract_partial_cap(c);
     const CUtensorMapDataType u8 = CU_TENSOR_MAP_DATA_TYPE_UINT8, f32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     cudaFuncSetAttribute(ls_i8_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
@@ -806,16 +807,9 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
         const size_t stage_b = off_o + sizeof(int) * noff;
         if ((rc = ensure(c, c->partial, sizeof(double) * (size_t)used, "partial lag tiles"))) return rc;
         if ((rc = ensure(c, c->jobdesc, stage_b, "job list"))) return rc;
-        // the staging area may still feed the previous launch's upload
-        if ((rc = cuda_check(c, cudaStreamSynchronize(c->stream), "job staging"))) return rc;
-        if (c->stage_bytes < stage_b) {
-            if (c->stage) cudaFreeHost(c->stage);
-            c->stage = nullptr;
-            c->stage_bytes = 0;
-            if ((rc = cuda_check(c, cudaHostAlloc(&c->stage, stage_b, cudaHostAllocDefault), "job staging"))) return rc;
-            c->stage_bytes = stage_b;
-        }
-        char *h = (char *)c->stage, *d = (char *)c->jobdesc.p;
+        void *staging;
+        if ((rc = job_stage(c, stage_b, &staging))) return rc;
+        char *h = (char *)staging, *d = (char *)c->jobdesc.p;
         I8Desc *hd = (I8Desc *)h;
         int *hg = (int *)(h + off_g), *ho = (int *)(h + off_o);
         std::vector<LsReduceJob> red;
@@ -869,6 +863,7 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
         std::copy(units.begin(), units.end(), (LsUnit *)(h + off_u));
         if ((rc = cuda_check(c, cudaMemcpyAsync(d, h, stage_b, cudaMemcpyHostToDevice, c->stream), "job list upload")))
             return rc;
+        if ((rc = job_stage_sent(c))) return rc;
         phase_begin(c, 1);
         const LsUnit *du = (const LsUnit *)(d + off_u);
         if (n4 > 0)
@@ -885,8 +880,15 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
         if ((rc = ls_reduce(c, red))) return rc;
         j0 = j1;
     }
-    int herr = 0;
-    if ((rc = cuda_check(c, cudaMemcpyAsync(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream),
+    return AMBER_OK;
+}
+
+int contract_i8_finish(amber_cuda_ctx *c)
+{
+    if (!c->i8_open) return AMBER_OK;
+    c->i8_open = false;
+    int rc, herr = 0;
+    if ((rc = cuda_check(c, cudaMemcpyAsync(&herr, c->misc.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream),
                          "error flag read")))
         return rc;
     if ((rc = cuda_check(c, cudaStreamSynchronize(c->stream), "contract_i8"))) return rc;
@@ -910,7 +912,8 @@ int contract_i8(amber_cuda_ctx *c, const DigitMaps &m1, const DigitMaps &m2, con
     jb.nanchors = (int)c->anchors.size();
     jb.mask_pass = false;
     jb.lag_out = lag_out;
-    return contract_i8_jobs(c, jobs);
+    const int rc = contract_i8_jobs(c, jobs);
+    return rc ? rc : contract_i8_finish(c);
 }
 
 }  // namespace amber

@@ -201,17 +201,17 @@ extern "C" int amber_cuda_cyl_bs(amber_cuda_ctx *c, const amber_cuda_cylbs_param
                                                 c->stream), "cyl_bs upload")))
             return rc;
     }
-    const double *res = (const double *)c->results.p;  // [ntri][2][ncsize]
+    const double *res = (const double *)c->results.p;  // [2][ntri][ncsize]
     const double L = (double)N * p->dnu_mhz * p->rc_prime;
     const double scale = pow(p->rc, 4.0) * L * L;
     for (int t0 = 0; t0 < ntri; t0 += batch) {
         const int nb = std::min(batch, ntri - t0);
-        const double *num = res + (size_t)t0 * 2 * ncsize;
-        const double *den = p->denominator == 0 ? aux : num + ncsize;
-        const long den_stride = p->denominator == 0 ? 0 : 2 * ncsize;
+        const double *num = res + (size_t)t0 * ncsize;
+        const double *den = p->denominator == 0 ? aux : num + (size_t)ntri * ncsize;
+        const long den_stride = p->denominator == 0 ? 0 : ncsize;
         const double *inv = tri_div ? aux + inv_off + t0 : nullptr;
         cylbs_fold<<<dim3((unsigned)(((long)M * N + kT - 1) / kT), nb), kT, 0, c->stream>>>(
-            num, 2 * ncsize, den, den_stride, inv, nc10, ncut, 1.0 / p->mabs_norm, d_win, d);
+            num, ncsize, den, den_stride, inv, nc10, ncut, 1.0 / p->mabs_norm, d_win, d);
         cylbs_rows<<<dim3((unsigned)((N + kT - 1) / kT), M, nb), kT, sizeof(double2) * N, c->stream>>>(d, M, N, tw, X);
         cylbs_cols<<<dim3((unsigned)((N + kT - 1) / kT), N, nb), kT, sizeof(double2) * N, c->stream>>>(X, M, N, tw,
                                                                                                       scale, o);

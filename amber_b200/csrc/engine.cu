@@ -72,7 +72,8 @@ struct Request {
     RunState run;
     bool started = false;
     // results (host)
-    std::vector<double> rdata, bldnu, numtri, cyl_out;
+    std::vector<double> rdata, cyl_out;
+    std::unique_ptr<double[]> bldnu, numtri;
     std::vector<int64_t> counts;
     double t_enqueue = 0, t_admit = 0, t_done = 0;
 };
@@ -163,17 +164,8 @@ void Engine::fail_req(Request *r, int rc, const std::string &msg)
 
 int Engine::setup(Request *r)
 {
-    amber_cuda_opts o;
-    amber_cuda_default_opts(&o);
-    o.device = owner->device;
-    o.precision = owner->fp64_abs ? AMBER_PREC_FP64_ABS : owner->precision;
-    o.hbm_budget = r->footprint;
-    o.stream = owner->stream;
-    o.chunk_px = owner->chunk_px;
-    int rc = amber_cuda_create(&o, &r->sub);
-    if (rc) return rc;
-    amber_cuda_ctx *s = r->sub;
-    s->contracts_elsewhere = owner->precision == AMBER_PREC_MIXED;
+    amber_cuda_ctx *s = r->sub = child_context(owner, r->footprint);
+    int rc;
     if ((rc = r->d_re_im ? amber_cuda_load_grid_device(s, r->N1, r->nc, r->Du, r->flag_key, r->d_re_im, r->d_ntig)
                          : amber_cuda_load_grid_packed(s, r->N1, r->nc, r->Du, r->flag_key, r->re_im.data(),
                                                        r->ntig.data())))
@@ -200,25 +192,24 @@ void Engine::finish(Request *r)
     amber_cuda_ctx *s = r->sub;
     const int ntri = (int)r->tri.size() / 3;
     const long ncsize = (long)(2 * r->nc10 + 1) * (2 * r->nc10 + 1);
-    std::vector<double> res((size_t)2 * ncsize * std::max(1, ntri));
+    // straight into the request's own buffers, which the copies touch first (no zero fill before)
+    const size_t n = (size_t)ncsize * ntri;
     int rc = AMBER_OK;
-    if (ntri > 0)
-        rc = cuda_check(s, cudaMemcpyAsync(res.data(), s->results.p, sizeof(double) * res.size(), cudaMemcpyDeviceToHost,
-                                           s->stream),
+    r->bldnu.reset(new double[std::max<size_t>(n, 1)]);
+    if (r->want_v2) r->numtri.reset(new double[std::max<size_t>(n, 1)]);
+    if (ntri > 0) {
+        const double *res = (const double *)s->results.p;
+        rc = cuda_check(s, cudaMemcpyAsync(r->bldnu.get(), res, sizeof(double) * n, cudaMemcpyDeviceToHost, s->stream),
                         "results download");
+        if (!rc && r->want_v2)
+            rc = cuda_check(s, cudaMemcpyAsync(r->numtri.get(), res + n, sizeof(double) * n, cudaMemcpyDeviceToHost,
+                                               s->stream),
+                            "results download");
+    }
     if (!rc) rc = cuda_check(s, cudaStreamSynchronize(s->stream), "results download");
     if (rc) {
         fail_req(r, rc, s->err);
         return;
-    }
-    r->bldnu.resize((size_t)ncsize * ntri);
-    if (r->want_v2) r->numtri.resize((size_t)ncsize * ntri);
-    for (int t = 0; t < ntri; ++t) {
-        std::copy(res.begin() + (size_t)t * 2 * ncsize, res.begin() + (size_t)t * 2 * ncsize + ncsize,
-                  r->bldnu.begin() + (size_t)t * ncsize);
-        if (r->want_v2)
-            std::copy(res.begin() + (size_t)t * 2 * ncsize + ncsize, res.begin() + (size_t)(t + 1) * 2 * ncsize,
-                      r->numtri.begin() + (size_t)t * ncsize);
     }
     if (r->want_cyl && ntri > 0) {
         // the reference's analysis chains: v1 files are read back divided by Num
@@ -231,8 +222,8 @@ void Engine::finish(Request *r)
             }
         s->last_ntri = ntri;
         s->last_v2 = r->want_v2;
-        const long n = 2 * (r->nc10 + 1 - r->cyl.n_cut) - 1;
-        r->cyl_out.assign((size_t)ntri * n * n, 0.0);
+        const long nk = 2 * (r->nc10 + 1 - r->cyl.n_cut) - 1;
+        r->cyl_out.assign((size_t)ntri * nk * nk, 0.0);
         if ((rc = amber_cuda_cyl_bs(s, &r->cyl, num.empty() ? nullptr : num.data(), r->cyl_out.data()))) {
             fail_req(r, rc, s->err);
             return;
@@ -336,7 +327,9 @@ void Engine::loop()
         double tc = now_ms();
         if (!jobs.empty()) {
             const long before = owner->contractions, launched = owner->launches;
-            rc = contract_i8_jobs(owner, jobs);  // synchronises the stream
+            rc = contract_i8_jobs(owner, jobs);
+            if (!rc) rc = contract_i8_finish(owner);
+            else owner->i8_open = false;
             launches += owner->contractions - before;
             all_launches += owner->launches - launched;
             for (size_t i = 0; i < owner->phase_used; ++i)
@@ -514,8 +507,8 @@ int amber_cuda_result(amber_cuda_ctx *c, int64_t ticket, int max_tri, double *rd
     const int ntri = (int)r->tri.size() / 3;
     const size_t ncsize = (size_t)(2 * r->nc10 + 1) * (2 * r->nc10 + 1);
     if (rdata) std::copy(r->rdata.begin(), r->rdata.begin() + (size_t)4 * ntri, rdata);
-    if (bldnu) std::copy(r->bldnu.begin(), r->bldnu.end(), bldnu);
-    if (numtri && r->want_v2) std::copy(r->numtri.begin(), r->numtri.end(), numtri);
+    if (bldnu) std::copy_n(r->bldnu.get(), ncsize * ntri, bldnu);
+    if (numtri && r->want_v2) std::copy_n(r->numtri.get(), ncsize * ntri, numtri);
     if (numdnu)
         for (int t = 0; t < ntri; ++t) std::copy(r->counts.begin(), r->counts.end(), numdnu + (size_t)t * ncsize);
     if (cyl_bs && r->want_cyl) std::copy(r->cyl_out.begin(), r->cyl_out.end(), cyl_bs);
