@@ -93,7 +93,7 @@ constexpr int NSET = NFORM / 4;              // former sets: each anchor group i
 constexpr int ABUF_COLS = 24;                // A buffer: 3 digits × 8 columns (32 int8 per row per digit)
 constexpr int ABUF4_COLS = 32;               // with four digits
 constexpr int NABUF_MAX = 8;                 // A buffers: as many as TMEM holds beside the accumulators
-constexpr long MIN_GROUPS = 5;                // least work of a unit (lagspace.cuh): ~10 µs
+constexpr long MIN_GROUPS = 4;                // least work of a unit (lagspace.cuh): ~10 µs
 constexpr int NSTAGE_MAX = 8;                // stages: as many as shared memory holds
 static_assert(3 * LS_ROWS + 5 * ABUF_COLS <= TMEM_COLS, "TMEM: five A buffers beside the widest accumulators");
 static_assert(NSET <= 4, "a set may be one use of a buffer ahead of the tensor pipe, not two: sets ≤ buffers");
@@ -159,6 +159,13 @@ __device__ __forceinline__ void tmem_st16x8(uint32_t taddr, const uint32_t (&v)[
 {
     asm volatile("tcgen05.st.sync.aligned.16x128b.x2.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
                  "r"(v[2]), "r"(v[3])
+                 : "memory");
+}
+// 16 lanes × 16 columns: v, then w eight columns on
+__device__ __forceinline__ void tmem_st16x16(uint32_t taddr, const uint32_t (&v)[4], const uint32_t (&w)[4])
+{
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
+                 "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
                  : "memory");
 }
 
@@ -597,7 +604,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             for (; g < ngr; g += NSET) {
                 uint32_t word;
                 asm volatile("ld.shared.b32 %0, [%1];" : "=r"(word) : "r"(group0 + 16 * g));
-                word = __shfl_sync(0xffffffffu, word, 0);
                 const uint32_t row = word & 0xffffu, blocks = word >> (16 + q);  // 16 × first row, live blocks
                 const uint32_t col = a_col0 + lane_field + ab * (NS == 4 ? ABUF4_COLS : ABUF_COLS);
                 // 16-byte chunk c of a 128-byte-swizzled row lies at chunk c ^ (row & 7)
@@ -613,7 +619,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 }
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {  // TMEM lanes 16·half .. +15 of the warp's 32
-                    uint32_t w[NS][4];
+                    uint32_t w[NS][4];  // zeros where a block is dead: one initialisation beats an else branch each
+#pragma unroll
+                    for (int dd = 0; dd < NS; ++dd)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) w[dd][e] = 0u;
 #pragma unroll
                     for (int jj = 0; jj < 2; ++jj) {
                         const int j = 2 * half + jj;
@@ -636,17 +646,16 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                                     w[dd][2 * h + jj] =
                                         pack_low_bytes(ya[dd + D0].x, ya[dd + D0].y, yb[dd + D0].x, yb[dd + D0].y);
                             }
-                        } else {
-#pragma unroll
-                            for (int dd = 0; dd < NS; ++dd) w[dd][jj] = w[dd][2 + jj] = 0u;
                         }
                     }
                     if (half == 0) {
                         if (!mbar_wait_conv(&ab_empty[ab], abph, abort_flag, err, 36)) { ok = false; return; }
                         fence_after();
                     }
-#pragma unroll
-                    for (int dd = 0; dd < NS; ++dd) tmem_st16x8(col + ((uint32_t)(16 * half) << 16) + 8 * dd, w[dd]);
+                    const uint32_t tcol = col + ((uint32_t)(16 * half) << 16);
+                    tmem_st16x16(tcol, w[0], w[1]);
+                    if constexpr (NS == 4) tmem_st16x16(tcol + 16, w[2], w[3]);
+                    else tmem_st16x8(tcol + 16, w[2]);
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 fence_before();
