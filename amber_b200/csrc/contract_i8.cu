@@ -70,6 +70,8 @@
 
 #include <algorithm>
 #include <cmath>
+#include <map>
+#include <tuple>
 #include <type_traits>
 #include <vector>
 
@@ -110,14 +112,16 @@ struct alignas(64) I8Desc {
     CUtensorMap t3;  // w·D3 fp32 {k, nc}, box {32, span3}, 128B swizzle
     CUtensorMap t1;  // w·D1 fp32 {k, nc}, box {32, AB}
     CUtensorMap t2;  // D2 digits {16, nc, kp/16, 3}, box {16, span2, 2, 3}
-    const int *e1, *e2, *e3;        // block exponents
+    CUtensorMap t2b; // a pair's second D2 (the other triangle with the same D1 and D3)
+    const int *e1, *e2, *e2b, *e3;  // block exponents
+    long tile2;                     // doubles from a unit's partial tile to the pair's second one
     const int *groups, *group_off;  // anchor groups of every anchor block
     long k;
     int nc, nc10, nclen, ks, rs, AB, ts;
     int span3, span2;
     int mask;                       // sampling-mask maps: class 3 as well
     uint32_t tx_bytes;              // bytes one slice's three TMA boxes deliver
-    int nst, st_bytes, st_d1, st_d2;  // stages, bytes of one, offsets of its D1 rows and D2 digits (D3 first)
+    int nst, st_bytes, st_d1, st_d2, st_d2b;  // stages, bytes of one, offsets of its D1 rows and D2 digits (D3 first)
 };
 
 __device__ __forceinline__ float2 sub2(float2 a, float2 b)
@@ -276,9 +280,10 @@ struct IssueState {
 //   SW_D: the A buffer holds P0, P1, P2; the first thread runs classes 0 and 1, the second class 2.
 //   SW_CLASS3: P1, P2, P3; class 3 = P3·Q0 + P2·Q1 (first) + P1·Q2 (second, an accumulator of its own).
 //   SW_MASK4: P0 .. P3; the first thread runs classes 0 and 3, the second classes 1 and 2.
+//   SW_PAIR, SW_PAIR4: three or four digits; each thread runs every class of one of the pair's triangles.
 // The loop is kept to few instructions beside the MMAs: they wait for issue slots behind the formers of
 // the same SM partition.
-enum { SW_D, SW_CLASS3, SW_MASK4 };
+enum { SW_D, SW_CLASS3, SW_MASK4, SW_PAIR, SW_PAIR4 };
 
 template <bool SECOND, int SWEEP>
 __device__ __forceinline__ bool issue_item(IssueState &t, int nsl, uint64_t *st_full, uint64_t *st_empty,
@@ -293,7 +298,7 @@ __device__ __forceinline__ bool issue_item(IssueState &t, int nsl, uint64_t *st_
         uint32_t next = t.groups;
         for (uint32_t g = 0; g < t.ngr; ++g) {
             const uint32_t q0 = sd + e.x, q1 = q0 + t.ddig, q2 = q1 + t.ddig, qh = t.desc_hi;
-            const uint32_t d = t.acc + e.y, idesc = e.z, a = t.a_first + t.ab * (SWEEP == SW_MASK4 ? ABUF4_COLS : ABUF_COLS);
+            const uint32_t d = t.acc + e.y, idesc = e.z, a = t.a_first + t.ab * (SWEEP == SW_MASK4 || SWEEP == SW_PAIR4 ? ABUF4_COLS : ABUF_COLS);
             const uint32_t bar = t.bars + t.ab * 8;
             next += 16;
             e = lds_u128(next);
@@ -304,7 +309,11 @@ __device__ __forceinline__ bool issue_item(IssueState &t, int nsl, uint64_t *st_
             // the MMAs that may be the first into their accumulator, then the rest
             auto leading = [&](auto addc) {
                 constexpr int ADD = decltype(addc)::value;
-                if constexpr (SWEEP == SW_D && !SECOND) {
+                if constexpr (SWEEP == SW_PAIR || SWEEP == SW_PAIR4) {
+#pragma unroll
+                    for (int i = 0; i < (SWEEP == SW_PAIR4 ? 4 : 3); ++i)
+                        umma_i8<ADD>(d + i * t.nmma, a + 8 * i, q0, qh, idesc);
+                } else if constexpr (SWEEP == SW_D && !SECOND) {
                     umma_i8<ADD>(d, a, q0, qh, idesc);
                     umma_i8<ADD>(d + t.nmma, a + 8, q0, qh, idesc);
                 } else if constexpr (SWEEP == SW_D) {
@@ -324,7 +333,13 @@ __device__ __forceinline__ bool issue_item(IssueState &t, int nsl, uint64_t *st_
             if (first) leading(std::integral_constant<int, 0>());
             else leading(std::integral_constant<int, 1>());
             first = false;
-            if constexpr (SWEEP == SW_D && !SECOND) {
+            if constexpr (SWEEP == SW_PAIR || SWEEP == SW_PAIR4) {
+                constexpr int NC = SWEEP == SW_PAIR4 ? 4 : 3;
+#pragma unroll
+                for (int i = 1; i < NC; ++i) umma_i8<1>(d + i * t.nmma, a + 8 * (i - 1), q1, qh, idesc);
+#pragma unroll
+                for (int i = 2; i < NC; ++i) umma_i8<1>(d + i * t.nmma, a + 8 * (i - 2), q2, qh, idesc);
+            } else if constexpr (SWEEP == SW_D && !SECOND) {
                 umma_i8<1>(d + t.nmma, a, q1, qh, idesc);
             } else if constexpr (SWEEP == SW_D) {
                 umma_i8<1>(d, a + 8, q1, qh, idesc);
@@ -350,9 +365,20 @@ __device__ __forceinline__ bool issue_item(IssueState &t, int nsl, uint64_t *st_
 // Whether a mask job's four class accumulators and four four-digit A buffers fit TMEM at MMA width nmma (≤ 96).
 __host__ __device__ constexpr bool mask4_fits(int nmma) { return 4 * nmma + NSET * ABUF4_COLS <= TMEM_COLS; }
 
-// FOUR: the launch's jobs are mask jobs run in one SW_MASK4 sweep (a kernel of its own: sharing one with the
-// three-digit sweeps cost those 9 % in register spills).
-template <bool FOUR>
+// Whether two triangles' accumulators and the A buffers fit TMEM: N ≤ 64 (D maps) or 48 (mask maps).
+__host__ __device__ constexpr bool pair_fits(bool mask, int nmma)
+{
+    return mask ? 8 * nmma + NSET * ABUF4_COLS <= TMEM_COLS : 6 * nmma + NSET * ABUF_COLS <= TMEM_COLS;
+}
+
+// MODE of a launch's jobs, each a kernel of its own (sharing one cost the three-digit sweeps 9 % in register spills):
+//   JOB_D      D maps (SW_D), and mask maps too wide for the next (SW_D, SW_CLASS3);
+//   JOB_MASK4  mask maps in one SW_MASK4 sweep;
+//   JOB_PAIR, JOB_PAIR4  D or mask maps of two triangles with the same r1 and r3: they share the formed A
+//              operand, whose digits are what bounds a small window's kernel, and differ in D2.
+enum { JOB_D, JOB_MASK4, JOB_PAIR, JOB_PAIR4, JOB_MODES };
+
+template <int MODE>
 __global__ void __launch_bounds__(NTHREADS, 1)
     ls_i8_kernel(const I8Desc *__restrict__ jobs, const LsUnit *__restrict__ units, double *__restrict__ partial,
                  int *err)
@@ -384,9 +410,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     // accumulators and four four-digit buffers fit TMEM (SW_MASK4: N ≤ 96), else classes 0-2 and then class 3
     // from digits formed again (SW_D, SW_CLASS3).  One sweep with four digits takes 1.25 times a sweep with three
     // where two took 2.2 times (realisations of 24-97 channels).
-    const int sweeps = jd->mask && !FOUR ? 2 : 1;
-    constexpr int abuf_cols = FOUR ? ABUF4_COLS : ABUF_COLS, ncls = FOUR ? 4 : 3;
-    const int nabuf = min(NABUF_MAX, (TMEM_COLS - ncls * nmma) / abuf_cols);
+    constexpr bool FOUR = MODE == JOB_MASK4 || MODE == JOB_PAIR4, PAIR = MODE == JOB_PAIR || MODE == JOB_PAIR4;
+    const int sweeps = MODE == JOB_D && jd->mask ? 2 : 1;
+    constexpr int abuf_cols = FOUR ? ABUF4_COLS : ABUF_COLS, ncls = FOUR ? 4 : 3, nacc = PAIR ? 2 * ncls : ncls;
+    const int nabuf = min(NABUF_MAX, (TMEM_COLS - nacc * nmma) / abuf_cols);
     const int nst = jd->nst, st_bytes = jd->st_bytes;
     double *out = partial + u.tile;
 
@@ -451,7 +478,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t a_col0 = tmem + ncls * nmma;
+    const uint32_t a_col0 = tmem + nacc * nmma;
     const int ngr = *ngroups_s;
     bool ok = true;
     const long k = jd->k;
@@ -462,7 +489,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 
     if (ngr == 0) {
         // no anchor of the block has a channel in range: the partial tile is zero
-        for (int e = tid; e < LS_ROWS * ncols; e += NTHREADS) out[e] = 0.0;
+        for (int e = tid; e < LS_ROWS * ncols; e += NTHREADS) {
+            out[e] = 0.0;
+            if (PAIR) out[jd->tile2 + e] = 0.0;
+        }
     } else if (warp == WARP_TMA) {
         if (lane == 0) {
             const int row0_3 = c0 - nc10 + toff3, row0_2 = c0 - nc10 + toff2;
@@ -478,6 +508,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                         tma_load_2d(st, &jd->t3, &st_full[s], x, row0_3);
                         tma_load_2d(st + st_d1, &jd->t1, &st_full[s], x, c0);
                         tma_load_4d(st + st_d2, &jd->t2, &st_full[s], 0, row0_2, x / 16, 0);
+                        if (PAIR) tma_load_4d(st + jd->st_d2b, &jd->t2b, &st_full[s], 0, row0_2, x / 16, 0);
                         if (++s == nst) { s = 0; ph ^= 1; }
                     }
             if (!ok)
@@ -523,7 +554,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         t.nabuf = uni(nabuf);
         t.nst = uni(nst);
         const uint32_t lbo = uni(jd->span2) * 16;               // the second 16-pixel group of a digit
-        const uint64_t desc0 = smem_desc_plain(smem_u32(stages + uni(jd->st_d2)), lbo);
+        const uint64_t desc0 = smem_desc_plain(smem_u32(stages + uni(PAIR && second ? jd->st_d2b : jd->st_d2)), lbo);
         t.ddig = (2 * lbo) >> 4;
         t.desc_lo = (uint32_t)desc0;
         t.desc_hi = (uint32_t)(desc0 >> 32);
@@ -532,8 +563,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         t.flags = smem_u32(ab_flags);
         t.bars = smem_u32(ab_empty);
         const uint32_t tmem_u = uni((int)tmem);
-        t.acc = tmem_u + (second ? (FOUR ? 1 : 2) * t.nmma : 0);
-        t.a_first = tmem_u + ncls * t.nmma;
+        t.acc = tmem_u + (second ? (PAIR ? ncls : FOUR ? 1 : 2) * t.nmma : 0);
+        t.a_first = tmem_u + nacc * t.nmma;
         t.ab = t.seen = t.s = t.ph = 0;
         t.need = 4;
         if (elect_one()) {
@@ -543,7 +574,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     // the epilogue of the previous item has read the accumulators out
                     ok = mbar_wait(acc_empty, (ni & 1) ^ 1, abort_flag, err, 32);
                     const int nsl = nslices(b);
-                    if constexpr (FOUR) {
+                    if constexpr (PAIR) {
+                        if (ok)
+                            ok = issue_item<false, FOUR ? SW_PAIR4 : SW_PAIR>(t, nsl, st_full, st_empty, abort_flag, err);
+                    } else if constexpr (FOUR) {
                         if (ok)
                             ok = second ? issue_item<true, SW_MASK4>(t, nsl, st_full, st_empty, abort_flag, err)
                                         : issue_item<false, SW_MASK4>(t, nsl, st_full, st_empty, abort_flag, err);
@@ -667,7 +701,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             g -= ngr;
         };
         for (long b = u.b0; b < u.b1 && ok; ++b) {
-            const int E = jd->e1[b] + jd->e3[b] + jd->e2[b];
+            const int E13 = jd->e1[b] + jd->e3[b];
             for (int sw = 0; sw < sweeps && ok; ++sw, ++ni) {
                 for (int sl = 0; sl < nslices(b); ++sl) {
                     if (!mbar_wait_conv(&st_ready[s], ph, abort_flag, err, 35)) { ok = false; break; }
@@ -688,32 +722,37 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 // ---- epilogue: int32 class accumulators → FP64, added into the unit's partial tile ----
                 if (!mbar_wait_warp(acc_full, ni & 1, abort_flag, err, 37)) { ok = false; break; }
                 fence_after();
-                // one unit of the last class in the sums: 127^−2·254^−2 (classes 0-2) or 127^−2·254^−3
-                const double scale = ldexp(1.0, E) * (sw == 0 && !FOUR ? 1.0 / (16129.0 * 64516.0)
-                                                                       : 1.0 / (16129.0 * 16387064.0));
                 const bool first = b == u.b0 && sw == 0;
                 // this lane's accumulator row and anchor slot
                 const int r = row_of(32 * q + lane), a = ks > 1 ? r / rs : 0;
                 const bool row_ok = ks > 1 ? r < mrows && r - a * rs < nclen : r < mrows;
-                for (int cb = 8 * ps; cb < nmma; cb += 8 * NSET) {
-                    uint32_t v0[8], v1[8], v2[8], v3[8];
-                    tmem_ld8(tmem + lane_field + cb, v0);
-                    if (sw == 0) tmem_ld8(tmem + lane_field + nmma + cb, v1);
-                    tmem_ld8(tmem + lane_field + 2 * nmma + cb, v2);
-                    if (FOUR) tmem_ld8(tmem + lane_field + 3 * nmma + cb, v3);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (!row_ok) continue;
+                for (int tri = 0; tri < (PAIR ? 2 : 1); ++tri) {
+                    const int E = E13 + (tri ? jd->e2b : jd->e2)[b];
+                    // one unit of the last class in the sums: 127^−2·254^−2 (classes 0-2) or 127^−2·254^−3
+                    const double scale = ldexp(1.0, E) * (sw == 0 && !FOUR ? 1.0 / (16129.0 * 64516.0)
+                                                                           : 1.0 / (16129.0 * 16387064.0));
+                    const uint32_t acc = tmem + lane_field + tri * ncls * nmma;
+                    double *outt = out + (tri ? jd->tile2 : 0);
+                    for (int cb = 8 * ps; cb < nmma; cb += 8 * NSET) {
+                        uint32_t v0[8], v1[8], v2[8], v3[8];
+                        tmem_ld8(acc + cb, v0);
+                        if (sw == 0) tmem_ld8(acc + nmma + cb, v1);
+                        tmem_ld8(acc + 2 * nmma + cb, v2);
+                        if (FOUR) tmem_ld8(acc + 3 * nmma + cb, v3);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        if (!row_ok) continue;
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const int colx = cb + e - a;  // slot a of a packed tile: lag column = column − a
-                        if (colx < 0 || colx >= ncols) continue;
-                        long long V = (long long)(int)v0[e] + (long long)(int)v2[e];  // class 3 alone, in two parts
-                        if (sw == 0)
-                            V = (long long)(int)v0[e] * 64516LL + (long long)(int)v1[e] * 254LL + (long long)(int)v2[e];
-                        if (FOUR) V = V * 254LL + (long long)(int)v3[e];
-                        double *o = out + (long)colx * LS_ROWS + r;
-                        const double val = (double)V * scale;
-                        *o = first ? val : *o + val;
+                        for (int e = 0; e < 8; ++e) {
+                            const int colx = cb + e - a;  // slot a of a packed tile: lag column = column − a
+                            if (colx < 0 || colx >= ncols) continue;
+                            long long V = (long long)(int)v0[e] + (long long)(int)v2[e];  // class 3 alone, in two parts
+                            if (sw == 0)
+                                V = (long long)(int)v0[e] * 64516LL + (long long)(int)v1[e] * 254LL + (long long)(int)v2[e];
+                            if (FOUR) V = V * 254LL + (long long)(int)v3[e];
+                            double *o = outt + (long)colx * LS_ROWS + r;
+                            const double val = (double)V * scale;
+                            *o = first ? val : *o + val;
+                        }
                     }
                 }
                 fence_before();
@@ -770,41 +809,75 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
     c->i8_open = true;
     const size_t pcap = contract_partial_cap(c);
     const CUtensorMapDataType u8 = CU_TENSOR_MAP_DATA_TYPE_UINT8, f32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-    cudaFuncSetAttribute(ls_i8_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
-    cudaFuncSetAttribute(ls_i8_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+    static void (*const KERNELS[JOB_MODES])(const I8Desc *, const LsUnit *, double *, int *) = {
+        ls_i8_kernel<JOB_D>, ls_i8_kernel<JOB_MASK4>, ls_i8_kernel<JOB_PAIR>, ls_i8_kernel<JOB_PAIR4>};
+    for (auto kernel : KERNELS)
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+    // Items: a job, or two jobs that share D1 and D3 and fit a pair (how jobs are paired changes no result:
+    // every sum of digits is exact).  A pair has half the units of its two jobs, each with 1.3 times the work, so
+    // jobs are paired where they would make more than three units an SM apart: D maps of a 59-channel
+    // realisation 10.4 → 8.7 ms, half of them in pairs.
+    long apart = 0;
+    for (const I8Job &jb : jobs) apart += ls_shape(jb.nc, jb.nc10, jb.k, c->num_sms, MIN_GROUPS).units();
+    const bool pairing = apart > 3L * c->num_sms;
+    struct Item {
+        size_t a, b;  // b = a: no second job
+        int mode;
+    };
+    std::vector<Item> items;
+    {
+        std::map<std::tuple<const float *, const float *, bool, const std::vector<int> *>, size_t> open;  // awaiting a partner
+        for (size_t i = 0; i < jobs.size(); ++i) {
+            const I8Job &jb = jobs[i];
+            const int nmma = ls_shape(jb.nc, jb.nc10, jb.k, c->num_sms, MIN_GROUPS).cols(0);
+            const int mode = jb.mask_pass && mask4_fits(nmma) ? JOB_MASK4 : JOB_D;
+            if (pairing && pair_fits(jb.mask_pass, nmma)) {
+                const auto key = std::make_tuple(jb.m1.f32, jb.m3.f32, jb.mask_pass, jb.weight);
+                const auto it = open.find(key);
+                if (it != open.end() && jobs[items[it->second].a].k == jb.k && jobs[items[it->second].a].nc10 == jb.nc10) {
+                    items[it->second].b = i;
+                    items[it->second].mode = jb.mask_pass ? JOB_PAIR4 : JOB_PAIR;
+                    open.erase(it);
+                    continue;
+                }
+                open[key] = items.size();
+            }
+            items.push_back(Item{i, i, mode});
+        }
+    }
     size_t j0 = 0;
-    while (j0 < jobs.size()) {
-        // plan as many jobs as their partial tiles allow in one launch
+    while (j0 < items.size()) {
+        // plan as many items as their partial tiles allow in one upload
         std::vector<LsJobPlan> plans;
         long used = 0;  // doubles of partial tiles
         size_t j1 = j0;
-        for (; j1 < jobs.size(); ++j1) {
-            const I8Job &jb = jobs[j1];
+        for (; j1 < items.size(); ++j1) {
+            const I8Job &jb = jobs[items[j1].a];
             LsJobPlan p;
             ls_plan_job(p, jb.nc, jb.nc10, jb.k, *jb.weight, c->num_sms, MIN_GROUPS, ls_force_bpu(c->chunk_px));
-            if (j1 > j0 && sizeof(double) * (size_t)(used + p.s.units() * p.s.tile()) > pcap) break;
+            const long need = p.s.units() * p.s.tile() * (items[j1].b != items[j1].a ? 2 : 1);
+            if (j1 > j0 && sizeof(double) * (size_t)(used + need) > pcap) break;
             p.unit_base = used;
-            used += p.s.units() * p.s.tile();
+            used += need;
             plans.push_back(std::move(p));
         }
-        // the units of jobs that run in one four-class sweep, then the others: a launch each
+        // the units of each mode: a launch each
         std::vector<LsUnit> units;
-        size_t n4 = 0;
-        for (int four = 1; four >= 0; --four) {
-            const size_t begin = units.size();
+        size_t begin[JOB_MODES + 1];
+        for (int mode = 0; mode < JOB_MODES; ++mode) {
+            begin[mode] = units.size();
             for (size_t i = 0; i < plans.size(); ++i) {
                 const size_t first = units.size();
-                const bool mask = jobs[j0 + i].mask_pass;
-                if ((mask && mask4_fits(plans[i].s.cols(0))) != (four != 0)) continue;
+                if (items[j0 + i].mode != mode) continue;
                 ls_units(plans[i], (int)i, units);
-                if (mask && !four)
+                if (mode == JOB_D && jobs[items[j0 + i].a].mask_pass)
                     for (size_t q = first; q < units.size(); ++q) units[q].work *= 1.6;  // the class-3 sweep
             }
             // largest units first, so that the small ones fill the tail of the launch
-            std::stable_sort(units.begin() + begin, units.end(),
+            std::stable_sort(units.begin() + begin[mode], units.end(),
                              [](const LsUnit &a, const LsUnit &b) { return a.work > b.work; });
-            if (four) n4 = units.size();
         }
+        begin[JOB_MODES] = units.size();
         size_t ngroups = 0, noff = 0;
         for (const LsJobPlan &p : plans) {
             ngroups += p.groups.size();
@@ -824,7 +897,9 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
         std::vector<LsReduceJob> red;
         size_t gpos = 0, opos = 0;
         for (size_t i = 0; i < plans.size(); ++i) {
-            const I8Job &jb = jobs[j0 + i];
+            const Item &item = items[j0 + i];
+            const I8Job &jb = jobs[item.a], &jb2 = jobs[item.b];
+            const bool pair = item.b != item.a;
             const LsJobPlan &p = plans[i];
             const LsShape &s = p.s;
             I8Desc &x = hd[i];
@@ -840,8 +915,12 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
             const cuuint64_t dstr[3] = {16, (cuuint64_t)jb.nc * 16, (cuuint64_t)jb.nc * jb.kp};
             const cuuint32_t box2[4] = {16, (cuuint32_t)x.span2, 2, 3};
             if ((rc = encode(c, &x.t2, u8, 4, jb.m2.dig, ddims, dstr, box2, CU_TENSOR_MAP_SWIZZLE_NONE))) return rc;
+            if (pair && (rc = encode(c, &x.t2b, u8, 4, jb2.m2.dig, ddims, dstr, box2, CU_TENSOR_MAP_SWIZZLE_NONE)))
+                return rc;
             x.e1 = jb.m1.bexp;
             x.e2 = jb.m2.bexp;
+            x.e2b = jb2.m2.bexp;
+            x.tile2 = p.s.units() * p.s.tile();
             x.e3 = jb.m3.bexp;
             x.groups = (const int *)(d + off_g) + gpos;
             x.group_off = (const int *)(d + off_o) + opos;
@@ -854,20 +933,24 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
             x.AB = s.AB;
             x.ts = s.ts;
             x.mask = jb.mask_pass ? 1 : 0;
-            x.tx_bytes = (uint32_t)(x.span3 * 128 + s.AB * 128 + 3 * 2 * x.span2 * 16);
+            const int d2_bytes = 3 * 2 * x.span2 * 16;
+            x.tx_bytes = (uint32_t)(x.span3 * 128 + s.AB * 128 + (pair ? 2 : 1) * d2_bytes);
             // whole 8-row swizzle atoms for the fp32 rows; every part starts on a 1024-byte boundary.  The
             // formers read a slot's whole 8-row blocks (all LS_ROWS rows with one slot) from every anchor on,
             // past the tile's rows too.
             x.st_d1 = (s.AB - 1 + (s.k > 1 ? s.rs : LS_ROWS) + 7) / 8 * 1024;
             x.st_d2 = x.st_d1 + (s.AB + 7) / 8 * 1024;
-            x.st_bytes = x.st_d2 + (3 * 2 * x.span2 * 16 + 1023) / 1024 * 1024;
+            x.st_d2b = x.st_d2 + (d2_bytes + 1023) / 1024 * 1024;
+            x.st_bytes = pair ? x.st_d2b + (d2_bytes + 1023) / 1024 * 1024 : x.st_d2b;
             x.nst = std::min(NSTAGE_MAX, SMEM_STAGES / x.st_bytes);
             std::copy(p.groups.begin(), p.groups.end(), hg + gpos);
             for (size_t q = 0; q < p.group_off.size(); ++q) ho[opos + q] = p.group_off[q];
             gpos += p.groups.size();
             opos += p.group_off.size();
-            red.push_back(LsReduceJob{(const double *)c->partial.p + p.unit_base, jb.lag_out,
-                                      s.nclen, s.k, s.rs, s.T, s.ts, s.nab, s.V, s.tile()});
+            for (int q = 0; q < (pair ? 2 : 1); ++q)
+                red.push_back(LsReduceJob{(const double *)c->partial.p + p.unit_base + q * x.tile2,
+                                          q ? jb2.lag_out : jb.lag_out, s.nclen, s.k, s.rs, s.T, s.ts, s.nab, s.V,
+                                          s.tile()});
         }
         std::copy(units.begin(), units.end(), (LsUnit *)(h + off_u));
         if ((rc = cuda_check(c, cudaMemcpyAsync(d, h, stage_b, cudaMemcpyHostToDevice, c->stream), "job list upload")))
@@ -875,16 +958,15 @@ int contract_i8_jobs(amber_cuda_ctx *c, const std::vector<I8Job> &jobs)
         if ((rc = job_stage_sent(c))) return rc;
         phase_begin(c, 1);
         const LsUnit *du = (const LsUnit *)(d + off_u);
-        if (n4 > 0)
-            ls_i8_kernel<true><<<(unsigned)n4, NTHREADS, SMEM_BYTES, c->stream>>>((const I8Desc *)d, du,
-                                                                                 (double *)c->partial.p, d_err);
-        if (units.size() > n4)
-            ls_i8_kernel<false><<<(unsigned)(units.size() - n4), NTHREADS, SMEM_BYTES, c->stream>>>(
-                (const I8Desc *)d, du + n4, (double *)c->partial.p, d_err);
+        for (int mode = 0; mode < JOB_MODES; ++mode) {
+            const unsigned n = (unsigned)(begin[mode + 1] - begin[mode]);
+            if (n == 0) continue;
+            KERNELS[mode]<<<n, NTHREADS, SMEM_BYTES, c->stream>>>((const I8Desc *)d, du + begin[mode],
+                                                                  (double *)c->partial.p, d_err);
+            c->launches += 1;
+            c->contractions += 1;
+        }
         phase_end(c);
-        const int nl = (n4 > 0) + (units.size() > n4);
-        c->launches += nl;
-        c->contractions += nl;
         if ((rc = cuda_check(c, cudaGetLastError(), "ls_i8_kernel launch"))) return rc;
         if ((rc = ls_reduce(c, red))) return rc;
         j0 = j1;

@@ -111,3 +111,23 @@ def test_mixed_windows_against_the_fixed_point_restatement(nc, nc10, flagged):
             want = _fixed_point(m, w, nc10, classes)
             got = r[key].reshape(want.shape)
             assert np.abs(got - want).max() <= 1e-9 * np.abs(o[scale]).max(), (r["r1"], r["r2"], r["r3"], key)
+
+
+@pytest.mark.parametrize("nc,nc10,version", [(40, 19, 2), (24, 11, 2), (20, 19, 1), (33, 31, 2)])
+def test_paired_triangles_equal_single_ones(nc, nc10, version):
+    """Triangles with the same first and third ring may run as pairs on one formed operand; run one at a time they
+    never do.  The digit sums are exact either way, so the lag arrays are equal bit for bit."""
+    import amber_b200
+    real = synth.tiny(96, nc, seed=55 + nc, nbins=8, hi=44.0, nc10=nc10, flagged=[3])
+    with amber_b200.Estimator(precision="mixed") as est:
+        est.load_grid(real.gv, real.counts, real.du, real.flag_key)
+        est.set_rings(real.ulow, real.uhigh)
+        est.set_channels(real.nc10, real.uf_chans)
+        tri = est.calcr()[:, :3].astype(np.int32)
+        last = tri[tri[:, 0] == 7]  # one r1 group: its ten triangles share a launch, four of them in two pairs
+        bl, _, nt = est.triangles(last, want_v2=version == 2)
+        for i, t in enumerate(last):
+            one, _, none = est.triangles(t[None], want_v2=version == 2)
+            np.testing.assert_array_equal(bl[i], one[0])
+            if version == 2:
+                np.testing.assert_array_equal(nt[i], none[0])
