@@ -9,9 +9,10 @@
 // fragments of the FP64 tensor-core MMA mma.sync m16n8k8 (1024 FMAs per
 // instruction; the m8n8k4 shape reaches only about half the FP64 tensor rate).
 // Fragments outside an anchor's channel range are skipped: the kernel is bound by
-// the DMMA pipe (84 % busy with every fragment computed), and at nc10 = nc − 1 three
-// quarters of the fragments are empty, at nc10 = nc/2 − 1 two fifths (46 triangles of
-// 32 channels: 66.6 → 28.9 ms of kernel time).  Per stage of 16
+// the DMMA pipe (84 % busy with every fragment computed, 75 % now), and at nc10 =
+// nc − 1 three quarters of the fragments are empty, at nc10 = nc/2 − 1 two fifths (46
+// triangles of 32 channels: 66.6 → 18.6 ms of kernel time, units of at least four
+// group-blocks included).  Per stage of 16
 // pixels the CTA copies the channel rows its anchors touch — w·D1 of the anchor
 // block, w·D3 and w·D2 of the spans their windows cover — into shared memory
 // once (transposed, [pixel][channel]); then, for every anchor group, it forms

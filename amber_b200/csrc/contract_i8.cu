@@ -51,7 +51,7 @@
 //
 // What bounds it, and what it measured (one CTA per SM, cycles per anchor group
 // and 32-pixel slice on the Ng1 = 740 maps, 128 channels, nclen = 127; triangles
-// of that size took 6.14 ms each before and 3.65 ms now):
+// of that size took 6.14 ms each before and 3.5 ms now):
 //   * 932 before.  The six MMAs of a group need 384 cycles at N = 128 (N/2 each,
 //     42 at least), 312 over the channel range alone.  The issuing warp was the
 //     bound: an mbarrier wait per group, operands the compiler did not know to be
@@ -59,8 +59,8 @@
 //     formers.  Counts in place of barriers, one elected thread per issuing warp,
 //     operands from a table and two issuing warps took it to 362 with the formers'
 //     arithmetic switched off.
-//   * The formers are the bound now: ~290 instructions per warp and group at 64 %
-//     of the issue slots.  A packed FP32x2 op with three different 64-bit operands
+//   * 415 now, and the formers are the bound: ~240 instructions per warp and group at
+//     62 % of the issue slots.  A packed FP32x2 op with three different 64-bit operands
 //     costs 3.3 cycles against 1.0 for a scalar one and PRMT costs 2, so packed
 //     ops save issue slots rather than pipe time: all-scalar digits were 8 % slower.
 //   * Blocks of 8 rows outside the channel range are skipped (a quarter of them at

@@ -219,7 +219,7 @@ __device__ __forceinline__ void dmma(double (&c)[4], const double (&a)[4], doubl
 // every fourth tile of 16 x, half the columns each.  The A fragments (cos, sin of j·x) come from the twiddle table, at indices that
 // advance by 16·x mod Ng per step of 16 j, and serve RN column tiles.  Bound by the FP64 pipe for wide
 // rings and by the map stores for narrow ones.  On the FP64 cores with two FMAs per pixel and j, each fed by a
-// shared load of its own, fourteen rings of 128 channels on 740 × 740 pixels took 13.6 ms; now 3.0 ms.
+// shared load of its own, fourteen rings of 128 channels on 740 × 740 pixels took 13.6 ms; now 3.8 ms.
 constexpr int RC = 32;       // columns per CTA
 constexpr int RS = RC + 1;   // their stride in shared memory: odd, so that a fragment load is conflict-free
 constexpr int RN = RC / 16;  // column tiles (of 8) per warp

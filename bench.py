@@ -67,8 +67,8 @@ SINGLE = "single realisation: 256^2 grid, 128 channels (4 of every 32 flagged), 
 
 # DRAM bytes per lag-triple product of the int8 lag-space kernel (ls_i8_kernel), from one ncu capture
 # of a full launch (profiles/ls_i8_kernel_config2_one_triangle.txt): every staged map slice is read
-# once per unit, so traffic grows with the products of a launch.
-DRAM_BYTES_PER_PRODUCT = (493.735e6 + 26.335e6) / 4.436392352e11
+# once per unit and every unit writes a partial tile, so traffic grows with the products of a launch.
+DRAM_BYTES_PER_PRODUCT = (494.969e6 + 84.983e6) / 4.436392352e11
 CPU_SAMPLE_REALISATION = 3  # side 256, 116 channels: its last (largest-ring) triangle is ~15 s of reference CPU
 
 
