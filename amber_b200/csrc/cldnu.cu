@@ -17,9 +17,9 @@
 //
 // Kernels:
 //   cldnu_pairs  one CTA per (bin, 16×16 tile of (p, q) with q-tile >= p-tile):
-//                the bin's cells in double-buffered chunks of 32 in shared memory,
-//                2×2 (p, q) per thread, FP64, sums to P[b][p][q − p]; and one thread
-//                per (bin, channel) for no_b[p], usum_b[p];
+//                the bin's cells in chunks of 16 through four stages of shared memory,
+//                two p of one q per thread, FP64, sums to P[b][p][q − p]; in a diagonal
+//                tile one more warp adds no_b[p] and usum_b[p];
 //   cldnu_reduce one warp per (bin, Δ): Σ_p P[b][p][Δ] / no_b[p].
 // Work: 5 FP64 operations per (cell, pair); the bin's grid rows are read once
 // per tile pair.  Bound by the largest bin's chain of cells.
@@ -34,14 +34,17 @@ namespace amber {
 
 namespace {
 
-constexpr int kTile = 16;   // (p, q) tile of a CTA, 2 × 2 pairs a thread
-constexpr int kChunk = 32;  // cells per shared-memory stage
-constexpr int kThreads = 64;
+constexpr int kTile = 16;    // (p, q) tile of a CTA
+constexpr int kChunk = 16;   // cells per shared-memory stage
+constexpr int kStages = 4;
+constexpr int kPair = 128;   // threads that add pairs, two p of one q each
+constexpr int kThreads = kPair + 32;  // and a warp that adds a diagonal tile's counts
 
-// One stage: the chunk's cells for the tile's p channels (value and sampling weight) and q channels.
+// One stage: the chunk's cells for the tile's p channels (value and sampling weight) and q channels, and their U.
 struct Stage {
     double2 g1[kChunk][kTile], g2[kChunk][kTile];
     double w1[kChunk][kTile];
+    double u[kChunk];
 };
 
 // n bytes (16 or 8) from global to shared memory, or zeros when !in
@@ -53,39 +56,13 @@ __device__ __forceinline__ void copy_async(void *dst, const void *src, bool in)
                  : "memory");
 }
 
-// no_b[p] and usum_b[p] of one bin, one thread per channel, cells in index order.
-__device__ __forceinline__ void norm_channel(const double *__restrict__ mask, const int *__restrict__ cells,
-                                             const double *__restrict__ uu, int k0, int k1, long nc, long p, int &no,
-                                             double &usum)
-{
-    int n = 0;
-    double u = 0.0;
-    auto term = [&](double w, double uk) {
-        // no[tmp] += NTiG (int += double); the sampling mask is 0 or 1, for which the conversions drop out
-        n = w == 0.0 || w == 1.0 ? n + (w == 1.0) : (int)((double)n + w);
-        u = __dadd_rn(u, __dmul_rn(uk, w));
-    };
-    int k = k0;
-    for (; k + 16 <= k1; k += 16) {
-        double w[16], uk[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            w[i] = mask[(long)cells[k + i] * nc + p];
-            uk[i] = uu[k + i];
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) term(w[i], uk[i]);
-    }
-    for (; k < k1; ++k) term(mask[(long)cells[k] * nc + p], uu[k]);
-    no = n;
-    usum = u;
-}
-
-// P[b][p][q − p] = Σ_{cells in b} (Re_p·Re_q + Im_p·Im_q)·NTiG[p] for one tile of pairs, or (the last CTAs of a
-// bin's row) the bin's counts.  The cells of a pair are added one after another, so a bin's chain is as long as
-// its cells: the bins run largest first, in tiles small enough that the largest one's pairs lie on many SMs, with
-// the next chunk in flight.  256² cells, 128 channels, 15 bins: 3.95 ms in 32 × 32 tiles staged without overlap,
-// plus 1.24 ms for the counts in a launch of their own; 0.75 ms now, all in one launch.
+// P[b][p][q − p] = Σ_{cells in b} (Re_p·Re_q + Im_p·Im_q)·NTiG[p] for one tile of pairs, and in a diagonal tile
+// the bin's counts and ΣU of its channels.  The cells of a pair are added one after another, so a bin's chain is
+// as long as its cells: the bins run largest first, in tiles small enough that the largest one's pairs lie on many
+// SMs, a tile's warps on all four partitions of its SM, with three chunks of cells in flight.  256² cells, 128
+// channels, 15 bins (the largest has 19004 cells): 5.2 ms in 32 × 32 tiles staged without overlap and with the counts
+// in a launch of their own; 0.75 ms with the counts in CTAs of their own (a chain of mask loads of 75 cycles a
+// cell), two warps a tile and two stages; 0.55-0.68 ms now, the call 1.40 → 1.20 ms.
 __global__ void __launch_bounds__(kThreads) cldnu_pairs(const double2 *__restrict__ grid,
                                                         const double *__restrict__ mask,
                                                         const int *__restrict__ cells, const double *__restrict__ uu,
@@ -93,88 +70,96 @@ __global__ void __launch_bounds__(kThreads) cldnu_pairs(const double2 *__restric
                                                         int *__restrict__ no, double *__restrict__ usum,
                                                         double *__restrict__ P)
 {
-    __shared__ Stage st[2];
+    __shared__ Stage st[kStages];
     const int b = gridDim.y - 1 - blockIdx.y;  // log bins: the last holds the most cells
     const int k0 = bin_off[b], k1 = bin_off[b + 1];
-    int t = blockIdx.x - (int)((nc + kThreads - 1) / kThreads);
-    if (t < 0) {
-        const long p = (long)blockIdx.x * kThreads + threadIdx.x;
-        if (p < nc) norm_channel(mask, cells, uu, k0, k1, nc, p, no[(long)b * nc + p], usum[(long)b * nc + p]);
-        return;
-    }
     // t → (tp, tq), tq >= tp
-    int tp = 0;
+    int t = blockIdx.x, tp = 0;
     while (t >= ntile - tp) {
         t -= ntile - tp;
         ++tp;
     }
     const int tq = tp + t;
     const long p0 = (long)tp * kTile, q0 = (long)tq * kTile;
-    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
-    const int ch = threadIdx.x % kTile, kr = threadIdx.x / kTile;  // staging: channel, first cell of the chunk
-    constexpr int KR = kThreads / kTile, KN = kChunk / KR;
-    const bool pin = p0 + ch < nc, qin = q0 + ch < nc;
-    double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-    int cell[KN];
+    // pairs: q channel and first p channel; staging: channel and first cell of the chunk
+    const int ch = threadIdx.x % kTile, row = threadIdx.x / kTile;
+    constexpr int KR = kPair / kTile, KN = kChunk / KR;
+    const bool pairs = threadIdx.x < kPair, pin = p0 + ch < nc, qin = q0 + ch < nc;
+    const int lane = (int)threadIdx.x - kPair;  // of the counting warp
+    double acc[2] = {0.0, 0.0}, u = 0.0;
+    int n = 0, cell[KN];
     auto load_cells = [&](int kc) {
+        if (!pairs) return;
 #pragma unroll
-        for (int i = 0; i < KN; ++i) cell[i] = kc + kr + KR * i < k1 ? cells[kc + kr + KR * i] : -1;
+        for (int i = 0; i < KN; ++i) cell[i] = kc + row + KR * i < k1 ? cells[kc + row + KR * i] : -1;
     };
-    auto stage = [&](Stage &s) {
+    auto stage = [&](Stage &s, int kc) {
+        if (pairs) {
 #pragma unroll
-        for (int i = 0; i < KN; ++i) {
-            const int k = kr + KR * i;
-            const long at = (cell[i] >= 0 ? (long)cell[i] : 0) * nc;
-            const long ap = at + (pin ? p0 + ch : 0), aq = at + (qin ? q0 + ch : 0);
-            copy_async<16>(&s.g1[k][ch], grid + ap, cell[i] >= 0 && pin);
-            copy_async<16>(&s.g2[k][ch], grid + aq, cell[i] >= 0 && qin);
-            copy_async<8>(&s.w1[k][ch], mask + ap, cell[i] >= 0 && pin);
+            for (int i = 0; i < KN; ++i) {
+                const int k = row + KR * i;
+                const long at = (cell[i] >= 0 ? (long)cell[i] : 0) * nc;
+                const long ap = at + (pin ? p0 + ch : 0), aq = at + (qin ? q0 + ch : 0);
+                copy_async<16>(&s.g1[k][ch], grid + ap, cell[i] >= 0 && pin);
+                copy_async<16>(&s.g2[k][ch], grid + aq, cell[i] >= 0 && qin);
+                copy_async<8>(&s.w1[k][ch], mask + ap, cell[i] >= 0 && pin);
+            }
+        } else if (lane < kChunk) {
+            const bool in = kc + lane < k1;
+            copy_async<8>(&s.u[lane], uu + (in ? kc + lane : k0), in);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     if (k0 < k1) {
-        load_cells(k0);
-        stage(st[0]);
-        load_cells(k0 + kChunk);
+#pragma unroll
+        for (int i = 0; i < kStages - 1; ++i) {
+            load_cells(k0 + kChunk * i);
+            stage(st[i], k0 + kChunk * i);
+        }
+        load_cells(k0 + kChunk * (kStages - 1));
     }
     int cur = 0;
-    for (int kc = k0; kc < k1; kc += kChunk, cur ^= 1) {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();  // this chunk is in; every reader of the other stage is done
-        if (kc + kChunk < k1) {
-            stage(st[cur ^ 1]);
-            load_cells(kc + 2 * kChunk);
-        }
+    for (int kc = k0; kc < k1; kc += kChunk, cur = (cur + 1) % kStages) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+        __syncthreads();  // this chunk is in; every reader of the stage filled next is done
+        stage(st[(cur + kStages - 1) % kStages], kc + kChunk * (kStages - 1));
+        load_cells(kc + kChunk * kStages);
         const int nk = min(kChunk, k1 - kc);
         const Stage &s = st[cur];
+        if (pairs) {
 #pragma unroll 4
-        for (int k = 0; k < nk; ++k) {
-            double2 g1[2], g2[2];
-            double w1[2];
+            for (int k = 0; k < nk; ++k) {
+                const double2 g2 = s.g2[k][ch];
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                g1[i] = s.g1[k][ty + 8 * i];
-                w1[i] = s.w1[k][ty + 8 * i];
-                g2[i] = s.g2[k][tx + 8 * i];
-            }
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
+                for (int i = 0; i < 2; ++i) {
                     // numer = Re1·Re2 + Im1·Im2; numer *= NTiG; pksum += numer
-                    const double numer =
-                        __dmul_rn(__dadd_rn(__dmul_rn(g1[i].x, g2[j].x), __dmul_rn(g1[i].y, g2[j].y)), w1[i]);
-                    acc[i][j] = __dadd_rn(acc[i][j], numer);
+                    const double2 g1 = s.g1[k][row + KR * i];
+                    const double numer = __dmul_rn(__dadd_rn(__dmul_rn(g1.x, g2.x), __dmul_rn(g1.y, g2.y)),
+                                                   s.w1[k][row + KR * i]);
+                    acc[i] = __dadd_rn(acc[i], numer);
                 }
+            }
+        } else if (tp == tq && lane < kTile) {
+#pragma unroll 4
+            for (int k = 0; k < nk; ++k) {
+                // no[tmp] += NTiG (int += double); the mask is 0 or 1, for which the conversions drop out
+                const double w = s.w1[k][lane];
+                n = w == 0.0 || w == 1.0 ? n + (w == 1.0) : (int)((double)n + w);
+                u = __dadd_rn(u, __dmul_rn(s.u[k], w));
+            }
         }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (pairs) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const long p = p0 + ty + 8 * i, q = q0 + tx + 8 * j;
-            if (q >= p && q < nc) P[((long)b * nc + p) * nc + (q - p)] = acc[i][j];
+        for (int i = 0; i < 2; ++i) {
+            const long p = p0 + row + KR * i, q = q0 + ch;
+            if (q >= p && q < nc) P[((long)b * nc + p) * nc + (q - p)] = acc[i];
         }
+    } else if (tp == tq && lane < kTile && p0 + lane < nc) {
+        no[(long)b * nc + p0 + lane] = n;
+        usum[(long)b * nc + p0 + lane] = u;
+    }
 }
 
 // cldnu[b][Δ] = Σ_p binps(p, p + Δ), p ascending, binps = P / no_b[p] where the count is not zero: one warp
@@ -263,8 +248,8 @@ extern "C" int amber_cuda_cl_dnu(amber_cuda_ctx *c, int NB, double umin, double 
         return rc;
     const double2 *grid = (const double2 *)c->grid.p;
     const double *mask = (const double *)c->mask.p;
-    const unsigned nnorm = (unsigned)((nc + kThreads - 1) / kThreads), npair = (unsigned)(ntile * (ntile + 1) / 2);
-    cldnu_pairs<<<dim3(nnorm + npair, NB), kThreads, 0, s>>>(grid, mask, d_cells, d_uu, d_off, nc, ntile, no, usum, P);
+    const unsigned npair = (unsigned)(ntile * (ntile + 1) / 2);
+    cldnu_pairs<<<dim3(npair, NB), kThreads, 0, s>>>(grid, mask, d_cells, d_uu, d_off, nc, ntile, no, usum, P);
     // no / usum come back first; the Δ sums then reuse the usum slot (same stream, in order)
     std::vector<int> h_no((size_t)NB * nc);
     std::vector<double> h_usum((size_t)NB * nc);
