@@ -355,9 +355,12 @@ int run_next_batch(amber_cuda_ctx *c, RunState &st, std::vector<I8Job> *jobs)
     // The next batch of the group: triangles whose ring union fits the budget.
     size_t spare = c->budget > c->held ? c->budget - c->held : 0;
     spare += c->maps_d.bytes + c->maps_i.bytes + c->y.bytes;
-    // the partial tiles of the last contraction give way to maps: the mixed path's reserve below covers
-    // them, the FP64 path frees them when the maps need the room and takes what is left afterwards
-    if (!c->contracts_elsewhere) spare += c->partial.bytes;
+    // The buffer of the partial tiles, which also staged the grid upload, gives way to maps only where it is freed
+    // or already counted: the FP64 path frees it when the maps need the room and takes what is left afterwards;
+    // the mixed path's reserve below covers as much of it as a launch's tiles may take; split-BF16 keeps it.
+    if (prec == AMBER_PREC_FP64) spare += c->partial.bytes;
+    else if (prec == AMBER_PREC_MIXED && !c->contracts_elsewhere)
+        spare += std::min(c->partial.bytes, contract_partial_cap(c));
     const size_t reserve = map_reserve(c);
     const long cap_slots = (long)((spare > reserve ? spare - reserve : 0) /
                                   (map_slot_bytes(prec, g.ng, c->nc, want_v2) + 1));

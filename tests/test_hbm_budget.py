@@ -1,0 +1,53 @@
+"""Triangle runs near their HBM budget: ring maps come in as many batches as the budget asks for, whatever the
+context's buffers hold from the grid upload and from earlier runs, and the batches change no result."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+DU = 1.0
+MAP_BYTES = {"fp64": 8, "bf16x3": 4, "mixed": 7}  # per map value; the mixed path's also have block exponents
+
+
+def _grid(nn, nc, hi, seed):
+    """Random cells inside every ring (|U| < hi cells), nothing elsewhere."""
+    rng = np.random.default_rng(seed)
+    gv, counts = np.zeros((nn, nn // 2 + 1, nc), np.complex128), np.zeros((nn, nn // 2 + 1, nc))
+    rows = np.r_[0:hi + 1, nn - hi:nn]
+    shape = (len(rows), hi + 1, nc)
+    gv[rows, :hi + 1] = rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+    counts[rows, :hi + 1] = 1.0
+    return gv, counts
+
+
+def _slot(precision, ng, nc):
+    """Bytes of one ring slot of one map set, and of its share of the map builder's intermediate."""
+    kp = (ng * ng + 255) // 256 * 256
+    return MAP_BYTES[precision] * nc * kp + 8 * nc + 4 * (kp // 256 + 1), 16 * ng * (ng // 3 + 1) * nc
+
+
+def _estimator(precision, gv, counts, edges, nc10, budget=0):
+    import amber_b200
+    est = amber_b200.Estimator(precision=precision, hbm_budget=budget)
+    est.load_grid(gv, counts, DU, 0)
+    est.set_rings(edges[:-1], edges[1:])
+    est.set_channels(nc10)
+    return est
+
+
+@pytest.mark.parametrize("precision,nn,nc,reserve", [("bf16x3", 256, 128, 64), ("mixed", 512, 256, 64 + 512)])
+def test_batches_leave_out_the_staged_grid_upload(precision, nn, nc, reserve):
+    """The buffer a grid was staged in stays held: a budget with room for four and a half of a group's 24 rings
+    beside it runs the group in batches."""
+    gv, counts = _grid(nn, nc, 40, 5)
+    edges = np.linspace(4.0, 40.0, 25)
+    tri = np.array([(23, r, r) for r in range(24)], np.int32)
+    with _estimator(precision, gv, counts, edges, 7) as est:
+        want = est.triangles(tri)
+        maps, y = _slot(precision, est.ng1(23), nc)
+    budget = 2 * 24 * gv.size + (reserve + 2) * MB + 9 * (maps + y) // 2
+    with _estimator(precision, gv, counts, edges, 7, budget) as est:
+        got = est.triangles(tri)
+    np.testing.assert_array_equal(got[0], want[0])
+    np.testing.assert_array_equal(got[1], want[1])
