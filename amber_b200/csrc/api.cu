@@ -35,10 +35,10 @@ int cuda_check(amber_cuda_ctx *c, cudaError_t e, const char *what)
                 cudaGetErrorString(e));
 }
 
-int ensure(amber_cuda_ctx *c, DevBuf &b, size_t bytes, const char *what)
+int ensure(amber_cuda_ctx *c, DevBuf &b, size_t bytes, const char *what, bool exact)
 {
     if (bytes <= b.bytes) return AMBER_OK;
-    size_t want = std::max(bytes, b.bytes + b.bytes / 4);
+    size_t want = exact ? bytes : std::max(bytes, b.bytes + b.bytes / 4);
     if (c->held - b.bytes + want > c->budget) {
         want = bytes;
         if (c->held - b.bytes + want > c->budget)
@@ -275,6 +275,35 @@ static size_t map_reserve(const amber_cuda_ctx *c)
            (c->precision == AMBER_PREC_MIXED && !c->contracts_elsewhere ? contract_partial_cap(c) : 0);
 }
 
+// Bytes of the map builder's intermediate for these rings on an ng-point grid.
+static size_t y_bytes(const amber_cuda_ctx *c, long ng, const std::set<int> &rings)
+{
+    long jmax = 1;
+    for (int r : rings) jmax = std::max(jmax, std::min(ng / 3, (long)ceil(c->uhigh[r])));
+    return sizeof(double2) * rings.size() * (size_t)ng * jmax * c->nc;
+}
+
+// What a batch of rings asks of the map buffers (no mask maps: i = 0).
+struct MapNeed {
+    size_t d, i, y;
+};
+
+// Bytes the context holds once its map buffers are grown to `n`: one that is larger already stays as it is.
+static size_t held_with(const amber_cuda_ctx *c, const MapNeed &n)
+{
+    return c->held + std::max(n.d, c->maps_d.bytes) - c->maps_d.bytes + std::max(n.i, c->maps_i.bytes) -
+           c->maps_i.bytes + std::max(n.y, c->y.bytes) - c->y.bytes;
+}
+
+// Grows the map buffers to `n`, no further: slack would come out of what the budget leaves to the others.
+static int grow_maps(amber_cuda_ctx *c, const MapNeed &n)
+{
+    int rc;
+    if ((rc = ensure(c, c->maps_d, n.d, "ring maps", true))) return rc;
+    if ((rc = ensure(c, c->maps_i, n.i, "ring mask maps", true))) return rc;
+    return ensure(c, c->y, n.y, "map intermediate", true);
+}
+
 int run_begin(amber_cuda_ctx *c, RunState &st, int ntri, const int *tri, int want_v2)
 {
     if (!c || ntri < 0 || (ntri > 0 && !tri)) return AMBER_ERR_ARG;
@@ -303,25 +332,25 @@ int run_begin(amber_cuda_ctx *c, RunState &st, int ntri, const int *tri, int wan
         }
         it->tris.push_back(t);
     }
-    // The maps of the largest group at once, where the budget holds them: grown group by group they would be
-    // freed and allocated again for each.
-    size_t maps = 0, y = 0;
-    const int passes = want_v2 ? 2 : 1;
+    // The maps of the largest group at once, where the budget holds them beside all that is held already: grown
+    // group by group they would be freed and allocated again for each.  Without them the run goes in batches.
+    MapNeed need{0, 0, 0};
     for (const RunState::Group &g : st.groups) {
         std::set<int> rings;
         for (int t : g.tris) rings.insert(tri + 3 * t, tri + 3 * t + 3);
-        long jmax = 1;
-        for (int r : rings) jmax = std::max(jmax, std::min(g.ng / 3, (long)ceil(c->uhigh[r])));
-        maps = std::max(maps, slot_bytes(c->precision, g.ng, c->nc) * rings.size());
-        y = std::max(y, sizeof(double2) * rings.size() * (size_t)g.ng * jmax * c->nc);
+        need.d = std::max(need.d, slot_bytes(c->precision, g.ng, c->nc) * rings.size());
+        need.y = std::max(need.y, y_bytes(c, g.ng, rings));
     }
-    const size_t other = c->held - c->maps_d.bytes - c->maps_i.bytes - c->y.bytes;
-    if (other + passes * std::max(maps, std::max(c->maps_d.bytes, c->maps_i.bytes)) + std::max(y, c->y.bytes) +
-            map_reserve(c) <= c->budget) {
-        if ((rc = ensure(c, c->maps_d, maps, "ring maps"))) return rc;
-        if (want_v2 && (rc = ensure(c, c->maps_i, maps, "ring mask maps"))) return rc;
-        if ((rc = ensure(c, c->y, y, "map intermediate"))) return rc;
-    }
+    if (want_v2) need.i = need.d;
+    // a buffer that has to grow does so by a quarter at least (a caller's loop over ever larger maps), where there
+    // is room for that too
+    auto quarter = [](size_t n, const DevBuf &b) { return n > b.bytes ? std::max(n, b.bytes + b.bytes / 4) : n; };
+    const MapNeed roomy{quarter(need.d, c->maps_d), quarter(need.i, c->maps_i), quarter(need.y, c->y)};
+    const size_t reserve = map_reserve(c);
+    rc = AMBER_OK;
+    if (held_with(c, roomy) + reserve <= c->budget) rc = grow_maps(c, roomy);
+    else if (held_with(c, need) + reserve <= c->budget) rc = grow_maps(c, need);
+    if (rc) c->err.clear();
     return AMBER_OK;
 }
 
@@ -389,15 +418,21 @@ int run_next_batch(amber_cuda_ctx *c, RunState &st, std::vector<I8Job> *jobs)
     }
     ms.nslots = (int)ms.ring_of_slot.size();
     const size_t nvals = (size_t)ms.nslots * c->nc * kp;
-    if (prec == AMBER_PREC_FP64) {
-        const size_t other = c->held - c->maps_d.bytes - c->maps_i.bytes - c->y.bytes;
-        if (other + reserve + map_slot_bytes(prec, g.ng, c->nc, want_v2) * ms.nslots > c->budget) {
-            if ((rc = cuda_check(c, cudaStreamSynchronize(c->stream), "partial lag tiles"))) return rc;
-            release(c, c->partial);
+    // The FP64 path's partial tiles, and buffers of earlier batches and runs that are larger than this batch needs
+    // (mask maps in a run without them included), were counted as spare above: they are given back where they
+    // stand in the way.
+    MapNeed need{per_slot * ms.nslots, want_v2 ? per_slot * ms.nslots : 0, y_bytes(c, g.ng, rings)};
+    const size_t covered = prec == AMBER_PREC_MIXED ? std::min(c->partial.bytes, reserve - ((size_t)64 << 20)) : 0;
+    if (held_with(c, need) + reserve - covered > c->budget) {
+        if ((rc = cuda_check(c, cudaStreamSynchronize(c->stream), "ring maps"))) return rc;
+        if (prec == AMBER_PREC_FP64) release(c, c->partial);
+        if (held_with(c, need) + reserve - covered > c->budget) {
+            if (c->maps_d.bytes > need.d) release(c, c->maps_d);
+            if (c->maps_i.bytes > need.i) release(c, c->maps_i);
+            if (c->y.bytes > need.y) release(c, c->y);
         }
     }
-    if ((rc = ensure(c, c->maps_d, per_slot * ms.nslots, "ring maps"))) return rc;
-    if (want_v2 && (rc = ensure(c, c->maps_i, per_slot * ms.nslots, "ring mask maps"))) return rc;
+    if ((rc = grow_maps(c, need))) return rc;
     // carve one map set (D or I) out of its buffer
     auto carve = [&](void *base, MapJob &job, DigitMaps *dm_base) {
         char *p = (char *)base;

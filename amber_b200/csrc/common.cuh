@@ -126,7 +126,8 @@ void phase_end(amber_cuda_ctx *c);
 
 int fail(amber_cuda_ctx *c, int code, const char *fmt, ...);
 int cuda_check(amber_cuda_ctx *c, cudaError_t e, const char *what);
-int ensure(amber_cuda_ctx *c, DevBuf &b, size_t bytes, const char *what);
+// Grows a buffer to at least `bytes`: by a quarter at least where the budget allows it, or to just that (exact).
+int ensure(amber_cuda_ctx *c, DevBuf &b, size_t bytes, const char *what, bool exact = false);
 int twiddle_table(amber_cuda_ctx *c, long n, const double2 **out);
 // The next pinned staging buffer, free to write (waits for its last upload); job_stage_sent after enqueuing the
 // upload from it.
