@@ -317,7 +317,9 @@ int run_begin(amber_cuda_ctx *c, RunState &st, int ntri, const int *tri, int wan
     cudaSetDevice(c->device);
     const int nclen = 2 * c->nc10 + 1;
     const long ncsize = (long)nclen * nclen;
-    if ((rc = ensure(c, c->results, sizeof(double) * 2 * ncsize * std::max(1, ntri), "results"))) return rc;
+    rc = ensure(c, c->results, sizeof(double) * 2 * ncsize * std::max(1, ntri), "results");
+    if (!rc || !c->results.p) c->last_ntri = 0;  // the run overwrites the last one's lag arrays
+    if (rc) return rc;
     st = RunState();
     st.tri.assign(tri, tri + 3 * ntri);
     st.want_v2 = want_v2;

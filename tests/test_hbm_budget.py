@@ -70,3 +70,22 @@ def test_batches_count_the_mask_maps_of_an_earlier_run(precision, nn, nc, hi, re
     np.testing.assert_array_equal(got[1], want[1])
     # FP64 units depend on the room for partial tiles: other groupings of the same sums
     np.testing.assert_allclose(got[0], want[0], rtol=0, atol=1e-10 * np.abs(want[0]).max())
+
+
+def test_failed_run_leaves_no_results():
+    """A run refused for its arguments keeps the last run's results; one that failed on the device has none."""
+    import amber_b200
+    gv, counts = _grid(512, 16, 240, 7)
+    with _estimator("fp64", gv, counts, np.array([2.0, 6.0, 200.0, 240.0]), 3, 2 * 24 * gv.size + 84 * MB) as est:
+        one = est.triangles([(0, 0, 0)], want_v2=True)
+        with pytest.raises(amber_b200.AmberError):
+            est.run([(0, 0, 3)])
+        again = est.fetch(want_v2=True)
+        for a, b in zip(again, one):
+            np.testing.assert_array_equal(a, b)
+        with pytest.raises(amber_b200.AmberError):
+            est.run([(0, 0, 0), (2, 2, 2)])  # the second triangle's maps exceed the budget
+        assert est.last_run_shape()[0] == 0
+        assert len(est.fetch()[0]) == 0
+        with pytest.raises(amber_b200.AmberError):
+            est.cyl_bs(n_cut=1)
