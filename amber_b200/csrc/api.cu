@@ -92,8 +92,14 @@ int twiddle_table(amber_cuda_ctx *c, long n, const double2 **out)
         DevBuf b;
         int rc = ensure(c, b, sizeof(double2) * n, "twiddle table");
         if (rc) return rc;
-        rc = cuda_check(c, cudaMemcpy(b.p, h.data(), sizeof(double2) * n, cudaMemcpyHostToDevice), "twiddles");
-        if (rc) return rc;
+        // on the context's stream, as the kernels that read it are: a copy on the default stream may still be on its
+        // way when it returns, and a non-blocking stream does not wait for it.  The host table is staged at once.
+        rc = cuda_check(c, cudaMemcpyAsync(b.p, h.data(), sizeof(double2) * n, cudaMemcpyHostToDevice, c->stream),
+                        "twiddles");
+        if (rc) {
+            release(c, b);
+            return rc;
+        }
         it = c->twiddles.emplace(n, b).first;
     }
     *out = reinterpret_cast<const double2 *>(it->second.p);
@@ -739,12 +745,13 @@ int amber_cuda_set_channels(amber_cuda_ctx *c, int nc10, int uf_nc, const int *u
     if ((rc = ensure(c, c->d_weight, sizeof(int) * c->nc, "channel weights"))) return rc;
     if ((rc = ensure(c, c->d_anchors, sizeof(int) * std::max<size_t>(1, anchors.size()), "anchors"))) return rc;
     cudaSetDevice(c->device);
-    if ((rc = cuda_check(c, cudaMemcpy(c->d_weight.p, w.data(), sizeof(int) * c->nc, cudaMemcpyHostToDevice),
+    if ((rc = cuda_check(c, cudaMemcpyAsync(c->d_weight.p, w.data(), sizeof(int) * c->nc, cudaMemcpyHostToDevice,
+                                            c->stream),
                          "weights")))
         return rc;
     if (!anchors.empty() &&
-        (rc = cuda_check(c, cudaMemcpy(c->d_anchors.p, anchors.data(), sizeof(int) * anchors.size(),
-                                       cudaMemcpyHostToDevice),
+        (rc = cuda_check(c, cudaMemcpyAsync(c->d_anchors.p, anchors.data(), sizeof(int) * anchors.size(),
+                                            cudaMemcpyHostToDevice, c->stream),
                          "anchors")))
         return rc;
     c->nc10 = nc10;
