@@ -113,6 +113,13 @@ def test_mixed_windows_against_the_fixed_point_restatement(nc, nc10, flagged):
             assert np.abs(got - want).max() <= 1e-9 * np.abs(o[scale]).max(), (r["r1"], r["r2"], r["r3"], key)
 
 
+# Two tiles an axis whose first is 97 lags or wider: the mask maps' four accumulators do not fit beside their A buffers
+# (N = 112 and 128), so they run two sweeps, in tiles of 104 + 89 and of 128 + 123 lags.
+@pytest.mark.parametrize("nc,nc10,flagged", [(110, 96, [50]), (126, 125, None)])
+def test_mixed_windows_of_two_wide_tiles(nc, nc10, flagged):
+    test_mixed_windows_against_the_fixed_point_restatement(nc, nc10, flagged)
+
+
 @pytest.mark.parametrize("nc,nc10,version", [(40, 19, 2), (24, 11, 2), (20, 19, 1), (33, 31, 2)])
 def test_paired_triangles_equal_single_ones(nc, nc10, version):
     """Triangles with the same first and third ring may run as pairs on one formed operand; run one at a time they
