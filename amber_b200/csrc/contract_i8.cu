@@ -391,6 +391,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     uint64_t *acc_full = ab_empty + NABUF_MAX, *acc_empty = acc_full + 1, *drain = acc_empty + 1;
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(drain + NMMA);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    volatile int *issued = abort_flag + 1;  // slices whose copies the TMA warp has started
     int *ngroups_s = reinterpret_cast<int *>(smem + SM_FLAGS - 4);
     uint32_t *ab_flags = reinterpret_cast<uint32_t *>(smem + SM_FLAGS);
     uint4 *sgroups = reinterpret_cast<uint4 *>(smem + SM_GROUPS);
@@ -466,6 +467,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         mbar_init(acc_empty, NFORM);
         for (int s = 0; s < NMMA; ++s) mbar_init(&drain[s], 1);
         *abort_flag = 0;
+        *issued = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == WARP_MMA) {
@@ -511,10 +513,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                         if (PAIR) tma_load_4d(st + jd->st_d2b, &jd->t2b, &st_full[s], 0, row0_2, x / 16, 0);
                         if (++s == nst) { s = 0; ph ^= 1; }
                     }
-            if (!ok)
-                for (int q = max(0, ns - nst); q < ns; ++q)
-                    for (long long i = 0; i < WAIT_LIMIT && !mbar_try_wait(&st_full[q % nst], ((q / nst) & 1)); ++i)
-                        __nanosleep(100);
+            *issued = ns;
         }
     } else if (warp == WARP_SCALE) {
         // scales each stage's D1 rows by 127·2^−(E1+E3) once for every row that uses them
@@ -590,11 +589,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     }
                     if (ok) umma_commit_bar(smem_u32(acc_full));
                 }
-            if (!ok) {
-                uint64_t *dr = drain + (second ? 1 : 0);
-                umma_commit_bar(smem_u32(dr));
-                for (long long i = 0; i < WAIT_LIMIT && !mbar_try_wait(dr, 0); ++i) __nanosleep(100);
-            }
         }
         __syncwarp();
     } else {
@@ -764,6 +758,21 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 
     fence_before();
     __syncthreads();
+    if (*abort_flag) {
+        // A wait gave up.  Copies and MMAs still in flight, those of a role that had finished its own loop
+        // included, have to end before the shared memory and TMEM that they use go away.
+        if (warp == WARP_TMA && lane == 0) {
+            const int n = *issued, ring = jd->nst;
+            for (int q = max(0, n - ring); q < n; ++q)
+                for (long long i = 0; i < WAIT_LIMIT && !mbar_try_wait(&st_full[q % ring], ((q / ring) & 1)); ++i)
+                    __nanosleep(100);
+        } else if ((warp == WARP_MMA || warp == WARP_MMA2) && elect_one()) {  // the thread that issued them
+            uint64_t *dr = drain + (warp == WARP_MMA2 ? 1 : 0);
+            umma_commit_bar(smem_u32(dr));
+            for (long long i = 0; i < WAIT_LIMIT && !mbar_try_wait(dr, 0); ++i) __nanosleep(100);
+        }
+        __syncthreads();
+    }
     if (warp == WARP_MMA) {
         fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));

@@ -94,6 +94,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     uint64_t *drain = acc_full + 1;
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(drain + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    volatile int *copies = abort_flag + 1;  // stages whose copies the TMA warp has started
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -118,6 +119,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         mbar_init(acc_full, 1);
         mbar_init(drain, 1);
         *abort_flag = 0;
+        *copies = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == WARP_MMA) {
@@ -144,14 +146,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 tma_load_2d(hi + STAGE_B / 2, &tm_lo, &b_full[s], x, bbase);
                 ++issued;
             }
-            if (*abort_flag) {
-                // let our own copies land before the CTA's shared memory goes away
-                for (int it = max(0, issued - NSB); it < issued; ++it) {
-                    const int s = it % NSB;
-                    for (long long i = 0; i < WAIT_LIMIT && !mbar_try_wait(&b_full[s], (it / NSB) & 1); ++i)
-                        __nanosleep(100);
-                }
-            }
+            *copies = issued;
         }
     } else if (warp == WARP_MMA) {
         if (lane == 0) {
@@ -182,13 +177,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 umma_commit(&b_empty[sb]);
                 umma_commit(&a_empty[sa]);
             }
-            if (ok) {
-                umma_commit(acc_full);
-            } else {
-                // drain: wait until every MMA we issued has finished before TMEM is freed
-                umma_commit(drain);
-                for (long long i = 0; i < WAIT_LIMIT && !mbar_try_wait(drain, 0); ++i) __nanosleep(100);
-            }
+            if (ok) umma_commit(acc_full);
         }
     } else {
         // ---- A formation: warps 0-7 ----
@@ -293,6 +282,20 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 
     fence_before();
     __syncthreads();
+    if (*abort_flag) {
+        // A wait gave up.  Copies and MMAs still in flight, those of a role that had finished its own loop
+        // included, have to end before the shared memory and TMEM that they use go away.
+        if (warp == WARP_TMA && lane == 0) {
+            const int n = *copies;
+            for (int it = max(0, n - NSB); it < n; ++it)
+                for (long long i = 0; i < WAIT_LIMIT && !mbar_try_wait(&b_full[it % NSB], (it / NSB) & 1); ++i)
+                    __nanosleep(100);
+        } else if (warp == WARP_MMA && lane == 0) {
+            umma_commit(drain);
+            for (long long i = 0; i < WAIT_LIMIT && !mbar_try_wait(drain, 0); ++i) __nanosleep(100);
+        }
+        __syncthreads();
+    }
     if (warp == WARP_MMA) {
         fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
