@@ -511,7 +511,6 @@ int run_next_batch(amber_cuda_ctx *c, RunState &st, std::vector<I8Job> *jobs)
                 jb.k = k; jb.kp = kp;
                 jb.nc = (int)c->nc; jb.nc10 = c->nc10;
                 jb.weight = &c->weight;
-                jb.nanchors = (int)c->anchors.size();
                 jb.mask_pass = pass == 1;
                 jb.lag_out = lag;
                 jl->push_back(jb);
@@ -605,8 +604,6 @@ int amber_cuda_create(const amber_cuda_opts *opts, amber_cuda_ctx **out)
     }
     cudaEventCreate(&c->ev0);
     cudaEventCreate(&c->ev1);
-    cudaEventCreate(&c->tev0);
-    cudaEventCreate(&c->tev1);
     *out = c;
     return AMBER_OK;
 }
@@ -617,8 +614,8 @@ void amber_cuda_destroy(amber_cuda_ctx *c)
     amber::engine_shutdown(c);
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
-    DevBuf *bufs[] = {&c->grid, &c->mask, &c->d_weight, &c->d_anchors, &c->y, &c->maps_d, &c->maps_i,
-                      &c->partial, &c->results, &c->ring_lohi, &c->misc, &c->mixed_scratch, &c->lagred, &c->jobdesc, &c->lagtrial, &c->lsred};
+    DevBuf *bufs[] = {&c->grid, &c->mask, &c->d_weight, &c->y, &c->maps_d, &c->maps_i, &c->partial, &c->results,
+                      &c->misc, &c->mixed_scratch, &c->lagred, &c->jobdesc, &c->lsred};
     for (DevBuf *b : bufs) release(c, *b);
     for (amber_cuda_ctx::Stage &s : c->stage) {
         if (s.p) cudaFreeHost(s.p);
@@ -631,8 +628,6 @@ void amber_cuda_destroy(amber_cuda_ctx *c)
     }
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
-    if (c->tev0) cudaEventDestroy(c->tev0);
-    if (c->tev1) cudaEventDestroy(c->tev1);
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;
 }
@@ -743,16 +738,10 @@ int amber_cuda_set_channels(amber_cuda_ctx *c, int nc10, int uf_nc, const int *u
     }
     int rc;
     if ((rc = ensure(c, c->d_weight, sizeof(int) * c->nc, "channel weights"))) return rc;
-    if ((rc = ensure(c, c->d_anchors, sizeof(int) * std::max<size_t>(1, anchors.size()), "anchors"))) return rc;
     cudaSetDevice(c->device);
     if ((rc = cuda_check(c, cudaMemcpyAsync(c->d_weight.p, w.data(), sizeof(int) * c->nc, cudaMemcpyHostToDevice,
                                             c->stream),
                          "weights")))
-        return rc;
-    if (!anchors.empty() &&
-        (rc = cuda_check(c, cudaMemcpyAsync(c->d_anchors.p, anchors.data(), sizeof(int) * anchors.size(),
-                                            cudaMemcpyHostToDevice, c->stream),
-                         "anchors")))
         return rc;
     c->nc10 = nc10;
     c->last_ntri = 0;  // the results buffer is laid out for the previous lag width

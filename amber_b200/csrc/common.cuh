@@ -66,7 +66,7 @@ struct amber_cuda_ctx {
     std::vector<int> anchors;  // channels with weight > 0, ascending
     std::vector<int64_t> counts;  // closed-form numdnu, nclen²
     int64_t total_vcp = 0;
-    amber::DevBuf d_weight, d_anchors;
+    amber::DevBuf d_weight;
 
     // twiddle tables e^{2πik/N}, per N
     std::map<long, amber::DevBuf> twiddles;
@@ -77,12 +77,10 @@ struct amber_cuda_ctx {
     amber::DevBuf maps_i;   // I maps (v2)
     amber::DevBuf partial;  // per-anchor/k-split partial lag tiles
     amber::DevBuf results;  // FP64 lag arrays [2][ntri][nclen²]: D sums, then mask sums
-    amber::DevBuf ring_lohi;
     amber::DevBuf misc;
     amber::DevBuf mixed_scratch;
     amber::DevBuf lagred;  // two-pass lag reduction: per-group sums and compensations
     amber::DevBuf jobdesc; // contraction job descriptors and work items
-    amber::DevBuf lagtrial; // autotuner: lag array of a discarded trial run
     amber::DevBuf lsred;    // lag-space reduction: job descriptors
     // pinned host staging of the job descriptors: two in turn, so that a launch is prepared while the upload
     // of the one before is still to run
@@ -115,7 +113,6 @@ struct amber_cuda_ctx {
     double last_products = 0;
     float last_ms = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    cudaEvent_t tev0 = nullptr, tev1 = nullptr;  // autotuner trials
 };
 
 namespace amber {
@@ -157,9 +154,6 @@ struct MapJob {
 };
 int build_maps(amber_cuda_ctx *c, const MapJob &job);
 
-// FP64 contraction of one triangle into a lag array (device).
-int contract_fp64(amber_cuda_ctx *c, const double *m1, const double *m2, const double *m3, long k, long kp,
-                  double *lag_out);
 // One FP64 contraction job (one triangle's D or mask pass on the context's channels).
 struct F64Job {
     const double *m1, *m2, *m3;  // [nc][kp] maps of r1, r2, r3
@@ -178,15 +172,12 @@ struct DigitMaps {
     const int8_t *dig;                // [3][kp/16][nc][16] base-254 digits of f32
     const int *bexp;                  // [kp/256] block exponents
 };
-int contract_i8(amber_cuda_ctx *c, const DigitMaps &m1, const DigitMaps &m2, const DigitMaps &m3, long k, long kp,
-                double *lag_out);
 // One mixed-precision contraction job: one triangle's D or mask pass of one realisation.
 struct I8Job {
     DigitMaps m1, m2, m3;   // ring maps of r1, r2, r3 on the job's Ng1 grid
     long k, kp;             // pixels, row stride (a multiple of 256)
     int nc, nc10;           // the realisation's channel count and lag half-width
     const std::vector<int> *weight;  // host: channel multiplicities (the planner's anchor groups)
-    int nanchors;
     bool mask_pass;         // sampling-mask maps: four product digits (a second sweep for class 3)
     double *lag_out;        // device: FP64 lag array [nclen²]
 };
@@ -235,7 +226,6 @@ size_t contract_partial_cap(const amber_cuda_ctx *c);
 // run on a lag width (nullptr: they can).
 size_t cyl_bs_bytes(int nc10, int n_cut, int ntri);
 const char *cyl_bs_invalid(const amber_cuda_cylbs_params *p, int nc10, int have_mask_sums);
-// Σ_x a·b·c over n points (FP64, deterministic) into out[0].
 // calCR: Num of every triangle (r1, r2, r3 in tri) from the N1² mask maps [ring][n], into device out[t].
 int triple_sums(amber_cuda_ctx *c, const double *maps, long n, const std::vector<int> &tri, double *out);
 

@@ -414,12 +414,6 @@ int contract_fp64_jobs(amber_cuda_ctx *c, const std::vector<F64Job> &jobs)
     return AMBER_OK;
 }
 
-int contract_fp64(amber_cuda_ctx *c, const double *m1, const double *m2, const double *m3, long k, long kp,
-                  double *lag_out)
-{
-    return contract_fp64_jobs(c, {F64Job{m1, m2, m3, k, kp, lag_out}});
-}
-
 int triple_sums(amber_cuda_ctx *c, const double *maps, long n, const std::vector<int> &tri, double *out)
 {
     const int ntri = (int)tri.size() / 3;

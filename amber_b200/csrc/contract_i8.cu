@@ -996,24 +996,4 @@ int contract_i8_finish(amber_cuda_ctx *c)
     return AMBER_OK;
 }
 
-int contract_i8(amber_cuda_ctx *c, const DigitMaps &m1, const DigitMaps &m2, const DigitMaps &m3, long k, long kp,
-                double *lag_out)
-{
-    std::vector<I8Job> jobs(1);
-    I8Job &jb = jobs[0];
-    jb.m1 = m1;
-    jb.m2 = m2;
-    jb.m3 = m3;
-    jb.k = k;
-    jb.kp = kp;
-    jb.nc = (int)c->nc;
-    jb.nc10 = c->nc10;
-    jb.weight = &c->weight;
-    jb.nanchors = (int)c->anchors.size();
-    jb.mask_pass = false;
-    jb.lag_out = lag_out;
-    const int rc = contract_i8_jobs(c, jobs);
-    return rc ? rc : contract_i8_finish(c);
-}
-
 }  // namespace amber

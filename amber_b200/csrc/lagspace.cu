@@ -83,7 +83,6 @@ int LsShape::cols(int t2) const
 {
     return k > 1 ? round16(nclen + k - 1) : round16(std::min(ts, nclen - ts * t2));
 }
-int LsShape::lag_cols(int t2) const { return k > 1 ? nclen : std::min(ts, nclen - ts * t2); }
 
 LsShape ls_shape(int nc, int nc10, long k_px, int sms, long min_groups, long force_bpu)
 {

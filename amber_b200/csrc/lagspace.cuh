@@ -56,7 +56,6 @@ struct LsShape {
     int V;        // units per (tile pair, anchor block)
     int rows(int t3) const;  // accumulator rows used by tile t3
     int cols(int t2) const;  // MMA width N of tile t2 (multiple of 16)
-    int lag_cols(int t2) const;  // lag columns Δ2 of tile t2 (k > 1: nclen)
     int units() const { return T * T * nab * V; }
     long tile() const { return (long)LS_ROWS * std::min(ts, nclen); }  // doubles of one partial tile
 };
