@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kThreads) cldnu_pairs(const double2 *__restric
 
 // cldnu[b][Δ] = Σ_p binps(p, p + Δ), p ascending, binps = P / no_b[p] where the count is not zero: one warp
 // per (bin, Δ) divides 32 terms at a time, then adds them one after another.  Bound by the loads' latency:
-// one thread per (bin, Δ) had a dependent load, divide and add for each p.  256² cells, 128 channels, 16 bins:
+// one thread per (bin, Δ) had a dependent load, divide and add for each p.  256² cells, 128 channels, 15 bins:
 // 76 µs before, 7 µs now.
 __global__ void __launch_bounds__(32) cldnu_reduce(const double *__restrict__ P, const int *__restrict__ no, long nc,
                                                    double *__restrict__ cldnu)

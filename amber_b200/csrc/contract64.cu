@@ -11,8 +11,8 @@
 // Fragments outside an anchor's channel range are skipped: the kernel is bound by
 // the DMMA pipe (84 % busy with every fragment computed, 75 % now), and at nc10 =
 // nc − 1 three quarters of the fragments are empty, at nc10 = nc/2 − 1 two fifths (46
-// triangles of 32 channels: 66.6 → 18.6 ms of kernel time, units of at least four
-// group-blocks included).  Per stage of 16
+// triangles of 32 channels: 66.6 → 18.6 ms of kernel time, together with units of
+// one pixel block for small jobs).  Per stage of 16
 // pixels the CTA copies the channel rows its anchors touch — w·D1 of the anchor
 // block, w·D3 and w·D2 of the spans their windows cover — into shared memory
 // once (transposed, [pixel][channel]); then, for every anchor group, it forms

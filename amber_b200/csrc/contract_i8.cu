@@ -44,10 +44,12 @@
 // warps, each set a whole anchor group, warp w the TMEM lanes 32·(w mod 4) .. +31)
 // and run each block's epilogue; warp 16 streams the slices by TMA; warps 17 and
 // 18 issue the MMAs, one elected thread each, into accumulators of their own;
-// warp 19 scales the staged D1 rows.  Five or more A buffers let the formers run
-// ahead of the tensor pipe.  Every wait is bounded; on expiry the CTA raises an
-// error flag the host turns into AMBER_ERR_TIMEOUT, drains its own copies and
-// MMAs and frees TMEM.  No cluster launch and no multicast.
+// warp 19 scales the staged D1 rows.  Four to eight A buffers (as many as TMEM
+// holds beside the accumulators; four are left at N = 96 and 48 of the four-digit
+// modes, one for each set of formers) let the formers run ahead of the tensor
+// pipe.  Every wait is bounded; on expiry the CTA raises an error flag the host
+// turns into AMBER_ERR_TIMEOUT, drains its copies and MMAs after its last barrier
+// and frees TMEM.  No cluster launch and no multicast.
 //
 // What bounds it, and what it measured (one CTA per SM, cycles per anchor group
 // and 32-pixel slice on the Ng1 = 740 maps, 128 channels, nclen = 127; triangles
@@ -95,7 +97,7 @@ constexpr int NSET = NFORM / 4;              // former sets: each anchor group i
 constexpr int ABUF_COLS = 24;                // A buffer: 3 digits × 8 columns (32 int8 per row per digit)
 constexpr int ABUF4_COLS = 32;               // with four digits
 constexpr int NABUF_MAX = 8;                 // A buffers: as many as TMEM holds beside the accumulators
-constexpr long MIN_GROUPS = 4;                // least work of a unit (lagspace.cuh): ~10 µs
+constexpr long MIN_GROUPS = 4;                // least work of a unit (lagspace.cuh): two blocks of a single anchor group
 constexpr int NSTAGE_MAX = 8;                // stages: as many as shared memory holds
 static_assert(3 * LS_ROWS + 5 * ABUF_COLS <= TMEM_COLS, "TMEM: five A buffers beside the widest accumulators");
 static_assert(NSET <= 4, "a set may be one use of a buffer ahead of the tensor pipe, not two: sets ≤ buffers");

@@ -107,8 +107,8 @@ LsShape ls_shape(int nc, int nc10, long k_px, int sms, long min_groups, long for
     s.AB = std::min(widest, ((nc + s.nab - 1) / s.nab + s.k - 1) / s.k * s.k);
     s.nab = (nc + s.AB - 1) / s.AB;
     s.nblk = std::max<long>(1, (k_px + LS_BLOCK - 1) / LS_BLOCK);
-    // Units: about six per SM for a large job, so the last wave is short; each of at least min_groups
-    // anchor groups × blocks, so that a small job still spreads over the SMs: at eight blocks a unit, the
+    // Units: about six per SM for a large job, so the last wave is short; down to one block each (two where a block
+    // is a single anchor group) for a small one, so that it still spreads over the SMs: at eight blocks a unit, the
     // kernel of one 2304-pixel triangle of 16 channels (9 blocks) took 104 µs on two SMs, and the eight
     // launches of a 32-channel realisation's 46 triangles 4.0 ms against 2.4 ms at one block a unit.
     const long per_block = std::max(1, s.AB / s.k) + 2;

@@ -60,9 +60,9 @@ struct LsShape {
     long tile() const { return (long)LS_ROWS * std::min(ts, nclen); }  // doubles of one partial tile
 };
 
-// min_groups: least work of a unit in anchor groups × pixel blocks, a block's own cost counted as two groups
-// (a unit's start and its partial tile, written once and read once, against its work); force_bpu > 0: exactly
-// that many blocks per unit (the last unit of a job may hold fewer)
+// min_groups: least work of a unit, in anchor groups × pixel blocks with a block's own cost counted as two groups.
+// With the values in use it asks for more than one block only where an anchor block is a single group (4: two
+// blocks); 1 asks for nothing.  force_bpu > 0: exactly that many blocks per unit (a job's last unit may hold fewer)
 LsShape ls_shape(int nc, int nc10, long k_px, int sms, long min_groups, long force_bpu = 0);
 
 // Blocks per unit that a chunk_px option asks for (0 = chosen by the planner)
@@ -98,7 +98,8 @@ struct LsReduceJob {
     long tile;              // doubles of one partial tile
 };
 // lag = Σ over units (and slots) of the partial tiles, compensated, fixed order; one launch for
-// every job of a contraction launch.  The descriptors are copied into the context's job staging.
+// every job of a contraction launch.  The descriptors are uploaded from the caller's (pageable) list into a buffer of
+// their own.
 int ls_reduce(amber_cuda_ctx *c, const std::vector<LsReduceJob> &jobs);
 
 }  // namespace amber

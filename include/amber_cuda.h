@@ -150,8 +150,8 @@ AMBER_API int amber_cuda_last_run_stats(const amber_cuda_ctx *ctx, double *produ
  * reference times only the whole loop (amber.c:230,285). */
 /* Shape of the results the last amber_cuda_triangles_run left on the device
  * (what _fetch and amber_cuda_cyl_bs read): its triangle count (0 once the
- * channels are set again or calCR has reused the buffer), the lag width nclen
- * and whether it holds the v2 mask sums. */
+ * channels are set again, calCR has reused the buffer or a run has failed on
+ * the device), the lag width nclen and whether it holds the v2 mask sums. */
 AMBER_API int amber_cuda_last_run_shape(const amber_cuda_ctx *ctx, int *ntri, int *nclen, int *v2);
 AMBER_API int amber_cuda_last_run_breakdown(const amber_cuda_ctx *ctx, double *ms_maps, double *ms_contract,
                                             double *ms_reduce, long *kernel_launches, long *contract_launches);
