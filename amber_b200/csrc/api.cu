@@ -392,15 +392,21 @@ int run_next_batch(amber_cuda_ctx *c, RunState &st, std::vector<I8Job> *jobs)
     // The next batch of the group: triangles whose ring union fits the budget.
     size_t spare = c->budget > c->held ? c->budget - c->held : 0;
     spare += c->maps_d.bytes + c->maps_i.bytes + c->y.bytes;
-    // The buffer of the partial tiles, which also staged the grid upload, gives way to maps only where it is freed
+    // The buffer of the partial tiles, which also staged the grid upload, gives way to maps only as far as it is freed
     // or already counted: the FP64 path frees it when the maps need the room and takes what is left afterwards;
-    // the mixed path's reserve below covers as much of it as a launch's tiles may take; split-BF16 keeps it.
-    if (prec == AMBER_PREC_FP64) spare += c->partial.bytes;
-    else if (prec == AMBER_PREC_MIXED && !c->contracts_elsewhere)
-        spare += std::min(c->partial.bytes, contract_partial_cap(c));
+    // the mixed path's reserve below covers as much of it as a launch's tiles may take; split-BF16 keeps it.  The
+    // three rings of one triangle are tried with all of it counted before a run is refused: it is freed where even
+    // they do not fit beside it.
+    const size_t gives = prec == AMBER_PREC_FP64 ? c->partial.bytes
+                         : prec == AMBER_PREC_MIXED && !c->contracts_elsewhere
+                             ? std::min(c->partial.bytes, contract_partial_cap(c))
+                             : 0;
     const size_t reserve = map_reserve(c);
-    const long cap_slots = (long)((spare > reserve ? spare - reserve : 0) /
-                                  (map_slot_bytes(prec, g.ng, c->nc, want_v2) + 1));
+    auto slots = [&](size_t room) {
+        return (long)((room > reserve ? room - reserve : 0) / (map_slot_bytes(prec, g.ng, c->nc, want_v2) + 1));
+    };
+    const long cap_slots = std::max(slots(spare + gives),
+                                    std::min(3L, slots(spare + (c->contracts_elsewhere ? 0 : c->partial.bytes))));
     if (cap_slots < 3) return fail(c, AMBER_ERR_OOM, "maps of one triangle (Ng1=%ld) exceed the budget", g.ng);
     std::vector<int> batch;
     std::set<int> rings;
@@ -439,6 +445,7 @@ int run_next_batch(amber_cuda_ctx *c, RunState &st, std::vector<I8Job> *jobs)
             if (c->maps_i.bytes > need.i) release(c, c->maps_i);
             if (c->y.bytes > need.y) release(c, c->y);
         }
+        if (held_with(c, need) > c->budget && !c->contracts_elsewhere) release(c, c->partial);
     }
     if ((rc = grow_maps(c, need))) return rc;
     // carve one map set (D or I) out of its buffer

@@ -72,6 +72,21 @@ def test_batches_count_the_mask_maps_of_an_earlier_run(precision, nn, nc, hi, re
     np.testing.assert_allclose(got[0], want[0], rtol=0, atol=1e-10 * np.abs(want[0]).max())
 
 
+@pytest.mark.parametrize("precision", ["bf16x3", "mixed", "fp64"])
+def test_a_run_that_fits_fits_again(precision):
+    """The partial tiles a run leaves held do not turn the same run away: a budget for just over a triangle's rings."""
+    gv, counts = _grid(60, 86, 28, 8)
+    edges = np.array([2.0, 15.0, 28.0])
+    with _estimator(precision, gv, counts, edges, 42) as est:
+        maps, y = _slot(precision, est.ng1(1), 86)
+    budget = 2 * 24 * gv.size + (64 + 512 * (precision == "mixed") + 1) * MB + 31 * (maps + y) // 10
+    with _estimator(precision, gv, counts, edges, 42, budget) as est:
+        first = est.triangles([(1, 1, 0)])
+        again = est.triangles([(1, 1, 0)])
+    for a, b in zip(again, first):
+        np.testing.assert_array_equal(a, b)
+
+
 def test_failed_run_leaves_no_results():
     """A run refused for its arguments keeps the last run's results; one that failed on the device has none."""
     import amber_b200
