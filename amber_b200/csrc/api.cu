@@ -281,6 +281,14 @@ static size_t map_reserve(const amber_cuda_ctx *c)
            (c->precision == AMBER_PREC_MIXED && !c->contracts_elsewhere ? contract_partial_cap(c) : 0);
 }
 
+// Bytes by which the split-BF16 path's partial tiles have to grow for maps of k pixels, with a margin for its lists and
+// reduction (the other paths fit their tiles to what the maps leave).
+static size_t tiles_growth(const amber_cuda_ctx *c, long k)
+{
+    const size_t need = c->precision == AMBER_PREC_BF16X3 ? contract_bf16x3_partial_bytes(c, k) : 0;
+    return need > c->partial.bytes ? need - c->partial.bytes + ((size_t)16 << 20) : 0;
+}
+
 // Bytes of the map builder's intermediate for these rings on an ng-point grid.
 static size_t y_bytes(const amber_cuda_ctx *c, long ng, const std::set<int> &rings)
 {
@@ -343,18 +351,19 @@ int run_begin(amber_cuda_ctx *c, RunState &st, int ntri, const int *tri, int wan
     // The maps of the largest group at once, where the budget holds them beside all that is held already: grown
     // group by group they would be freed and allocated again for each.  Without them the run goes in batches.
     MapNeed need{0, 0, 0};
+    size_t reserve = map_reserve(c);
     for (const RunState::Group &g : st.groups) {
         std::set<int> rings;
         for (int t : g.tris) rings.insert(tri + 3 * t, tri + 3 * t + 3);
         need.d = std::max(need.d, slot_bytes(c->precision, g.ng, c->nc) * rings.size());
         need.y = std::max(need.y, y_bytes(c, g.ng, rings));
+        reserve = std::max(reserve, tiles_growth(c, g.ng * g.ng));
     }
     if (want_v2) need.i = need.d;
     // a buffer that has to grow does so by a quarter at least (a caller's loop over ever larger maps), where there
     // is room for that too
     auto quarter = [](size_t n, const DevBuf &b) { return n > b.bytes ? std::max(n, b.bytes + b.bytes / 4) : n; };
     const MapNeed roomy{quarter(need.d, c->maps_d), quarter(need.i, c->maps_i), quarter(need.y, c->y)};
-    const size_t reserve = map_reserve(c);
     rc = AMBER_OK;
     if (held_with(c, roomy) + reserve <= c->budget) rc = grow_maps(c, roomy);
     else if (held_with(c, need) + reserve <= c->budget) rc = grow_maps(c, need);
@@ -401,12 +410,14 @@ int run_next_batch(amber_cuda_ctx *c, RunState &st, std::vector<I8Job> *jobs)
                          : prec == AMBER_PREC_MIXED && !c->contracts_elsewhere
                              ? std::min(c->partial.bytes, contract_partial_cap(c))
                              : 0;
-    const size_t reserve = map_reserve(c);
+    const size_t reserve = map_reserve(c), growth = tiles_growth(c, k);
     auto slots = [&](size_t room) {
         return (long)((room > reserve ? room - reserve : 0) / (map_slot_bytes(prec, g.ng, c->nc, want_v2) + 1));
     };
-    const long cap_slots = std::max(slots(spare + gives),
-                                    std::min(3L, slots(spare + (c->contracts_elsewhere ? 0 : c->partial.bytes))));
+    long cap_slots = std::max(slots(spare + gives),
+                              std::min(3L, slots(spare + (c->contracts_elsewhere ? 0 : c->partial.bytes))));
+    // split-BF16 tiles that outgrow the reserve: fewer rings a batch, down to one triangle's
+    if (growth > reserve && cap_slots > 3) cap_slots = std::max(3L, slots(spare > growth ? spare - growth + reserve : 0));
     if (cap_slots < 3) return fail(c, AMBER_ERR_OOM, "maps of one triangle (Ng1=%ld) exceed the budget", g.ng);
     std::vector<int> batch;
     std::set<int> rings;
@@ -437,10 +448,11 @@ int run_next_batch(amber_cuda_ctx *c, RunState &st, std::vector<I8Job> *jobs)
     // stand in the way.
     MapNeed need{per_slot * ms.nslots, want_v2 ? per_slot * ms.nslots : 0, y_bytes(c, g.ng, rings)};
     const size_t covered = prec == AMBER_PREC_MIXED ? std::min(c->partial.bytes, reserve - ((size_t)64 << 20)) : 0;
-    if (held_with(c, need) + reserve - covered > c->budget) {
+    const size_t left = std::max(reserve - covered, growth);
+    if (held_with(c, need) + left > c->budget) {
         if ((rc = cuda_check(c, cudaStreamSynchronize(c->stream), "ring maps"))) return rc;
         if (prec == AMBER_PREC_FP64) release(c, c->partial);
-        if (held_with(c, need) + reserve - covered > c->budget) {
+        if (held_with(c, need) + left > c->budget) {
             if (c->maps_d.bytes > need.d) release(c, c->maps_d);
             if (c->maps_i.bytes > need.i) release(c, c->maps_i);
             if (c->y.bytes > need.y) release(c, c->y);

@@ -165,6 +165,8 @@ int contract_fp64_jobs(amber_cuda_ctx *c, const std::vector<F64Job> &jobs);
 // Split-BF16×3 contraction (tcgen05, FP32 accumulation in TMEM).
 int contract_bf16x3(amber_cuda_ctx *c, const uint16_t *h1, const uint16_t *l1, const uint16_t *h2,
                     const uint16_t *l2, const uint16_t *h3, const uint16_t *l3, long k, long kp, double *lag_out);
+// Bytes of its partial lag tiles for maps of k pixels.
+size_t contract_bf16x3_partial_bytes(const amber_cuda_ctx *c, long k);
 // Mixed-precision contraction: base-254 int8 digits on the tensor cores
 // (tcgen05 kind::i8, exact int32 accumulation in TMEM).
 struct DigitMaps {

@@ -348,37 +348,35 @@ int launch(amber_cuda_ctx *c, const CUtensorMap &th, const CUtensorMap &tl, cons
     return cuda_check(c, cudaGetLastError(), "contract_tc_kernel launch");
 }
 
-}  // namespace
-
-int contract_bf16x3(amber_cuda_ctx *c, const uint16_t *h1, const uint16_t *l1, const uint16_t *h2, const uint16_t *l2,
-                   const uint16_t *h3, const uint16_t *l3, long k, long kp, double *lag_out)
-{
-    const int nc10 = c->nc10, nclen = 2 * nc10 + 1;
-    const long ncsize = (long)nclen * nclen;
-    const int nA = (int)c->anchors.size();
-    if (nA == 0) return cuda_check(c, cudaMemsetAsync(lag_out, 0, sizeof(double) * ncsize, c->stream), "zero lag");
-
-    // tile plan
+// Tiles, anchor groups and pixel chunks of one triangle's contraction.
+struct TcPlan {
     int P, BN, MT, NT;
+    std::vector<Group> groups;
+    long nch, chunk;
+};
+
+TcPlan tc_plan(const amber_cuda_ctx *c, long k)
+{
+    TcPlan p;
+    const int nclen = 2 * c->nc10 + 1, nA = (int)c->anchors.size();
     if (nclen + 1 <= 128) {
-        P = 2;
-        BN = std::max(32, (nclen + 1 + 31) / 32 * 32);
-        MT = 1;
-        NT = 1;
+        p.P = 2;
+        p.BN = std::max(32, (nclen + 1 + 31) / 32 * 32);
+        p.MT = 1;
+        p.NT = 1;
     } else {
-        P = 1;
-        MT = (nclen + BM - 1) / BM;
-        NT = (nclen + 255) / 256;
-        BN = ((nclen + NT - 1) / NT + 31) / 32 * 32;
+        p.P = 1;
+        p.MT = (nclen + BM - 1) / BM;
+        p.NT = (nclen + 255) / 256;
+        p.BN = ((nclen + p.NT - 1) / p.NT + 31) / 32 * 32;
     }
     // anchor groups: consecutive unflagged channels pair up when P == 2
-    std::vector<Group> groups;
     for (int i = 0; i < nA;) {
         Group g{};
         g.p1[0] = c->anchors[i];
         g.aidx[0] = i;
         g.count = 1;
-        if (P == 2 && i + 1 < nA && c->anchors[i + 1] - c->anchors[i] <= BN - nclen) {
+        if (p.P == 2 && i + 1 < nA && c->anchors[i + 1] - c->anchors[i] <= p.BN - nclen) {
             g.p1[1] = c->anchors[i + 1];
             g.aidx[1] = i + 1;
             g.off1 = g.p1[1] - g.p1[0];
@@ -390,21 +388,47 @@ int contract_bf16x3(amber_cuda_ctx *c, const uint16_t *h1, const uint16_t *l1, c
             g.off1 = 0;
             i += 1;
         }
-        groups.push_back(g);
+        p.groups.push_back(g);
     }
-    const long base_items = (long)groups.size() * MT * NT;
+    const long base_items = std::max<long>(1, (long)p.groups.size() * p.MT * p.NT);
     const long target = 4L * c->num_sms;
     long max_chunk = c->chunk_px > 0 ? c->chunk_px : 32768;
     max_chunk = std::max<long>(KBLK, max_chunk / KBLK * KBLK);
-    long nch = std::max<long>((k + max_chunk - 1) / max_chunk, std::min<long>((target + base_items - 1) / base_items,
-                                                                           (k + 1023) / 1024));
-    nch = std::max<long>(nch, 1);
-    long chunk = ((k + nch - 1) / nch + KBLK - 1) / KBLK * KBLK;
-    nch = (k + chunk - 1) / chunk;
+    p.nch = std::max<long>((k + max_chunk - 1) / max_chunk, std::min<long>((target + base_items - 1) / base_items,
+                                                                         (k + 1023) / 1024));
+    p.nch = std::max<long>(p.nch, 1);
+    p.chunk = ((k + p.nch - 1) / p.nch + KBLK - 1) / KBLK * KBLK;
+    p.nch = (k + p.chunk - 1) / p.chunk;
+    return p;
+}
+
+size_t tc_partial_bytes(const amber_cuda_ctx *c, const TcPlan &p)
+{
+    const size_t nclen = 2 * (size_t)c->nc10 + 1;
+    return sizeof(double) * c->anchors.size() * (size_t)p.nch * nclen * nclen;
+}
+
+}  // namespace
+
+size_t contract_bf16x3_partial_bytes(const amber_cuda_ctx *c, long k) { return tc_partial_bytes(c, tc_plan(c, k)); }
+
+int contract_bf16x3(amber_cuda_ctx *c, const uint16_t *h1, const uint16_t *l1, const uint16_t *h2, const uint16_t *l2,
+                   const uint16_t *h3, const uint16_t *l3, long k, long kp, double *lag_out)
+{
+    const int nc10 = c->nc10, nclen = 2 * nc10 + 1;
+    const long ncsize = (long)nclen * nclen;
+    const int nA = (int)c->anchors.size();
+    if (nA == 0) return cuda_check(c, cudaMemsetAsync(lag_out, 0, sizeof(double) * ncsize, c->stream), "zero lag");
+
+    const TcPlan plan = tc_plan(c, k);
+    const int P = plan.P, BN = plan.BN, MT = plan.MT, NT = plan.NT;
+    const std::vector<Group> &groups = plan.groups;
+    const long nch = plan.nch, chunk = plan.chunk;
+    const long items = (long)groups.size() * MT * NT * nch;
 
     int rc;
     const size_t gbytes = sizeof(Group) * groups.size();
-    const size_t pbytes = sizeof(double) * (size_t)nA * nch * ncsize;
+    const size_t pbytes = tc_partial_bytes(c, plan);
     if ((rc = ensure(c, c->partial, pbytes, "partial lag tiles"))) return rc;
     if ((rc = ensure(c, c->misc, 256 + gbytes, "tile plan"))) return rc;
     int *d_err = (int *)c->misc.p;
@@ -426,8 +450,6 @@ int contract_bf16x3(amber_cuda_ctx *c, const uint16_t *h1, const uint16_t *l1, c
     prm.weight = (const int *)c->d_weight.p;
     prm.partial = (double *)c->partial.p;
     prm.err = d_err;
-    const long items = base_items * nch;
-
 #define CASE(PP, BB)                                                   \
     if (P == PP && BN == BB) rc = launch<PP, BB>(c, th, tl, prm, items); \
     else

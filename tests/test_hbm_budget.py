@@ -72,6 +72,21 @@ def test_batches_count_the_mask_maps_of_an_earlier_run(precision, nn, nc, hi, re
     np.testing.assert_allclose(got[0], want[0], rtol=0, atol=1e-10 * np.abs(want[0]).max())
 
 
+def test_maps_leave_room_for_the_split_bf16_tiles():
+    """Partial tiles larger than the reserve, beside them room for three of eight rings: batches, not all rings first."""
+    gv, counts = _grid(120, 64, 56, 9)
+    edges = np.linspace(4.0, 56.0, 9)
+    tri = np.array([(7, r, r) for r in range(8)], np.int32)
+    with _estimator("bf16x3", gv, counts, edges, 63) as est:
+        want = est.triangles(tri)
+        maps, y = _slot("bf16x3", est.ng1(7), 64)
+    tiles = 8 * 64 * 19 * 127 ** 2  # anchors, pixel chunks on 148 SMs, lag cells
+    budget = 24 * gv.size + tiles + 32 * MB + 32 * (maps + y) // 10
+    with _estimator("bf16x3", gv, counts, edges, 63, budget) as est:
+        got = est.triangles(tri)
+    np.testing.assert_array_equal(got[0], want[0])
+
+
 @pytest.mark.parametrize("precision", ["bf16x3", "mixed", "fp64"])
 def test_a_run_that_fits_fits_again(precision):
     """The partial tiles a run leaves held do not turn the same run away: a budget for just over a triangle's rings."""
